@@ -138,7 +138,8 @@ int mlora_lora_shrink(const void* d_x, int64_t ldx, const void* d_A_all, const i
  *   tile may still bump its arrival counter afterwards, the whole buffer must be zero-filled again
  *   before its next use (the word is sticky: the caller clears it). */
 size_t mlora_linear_workspace(int32_t T, int32_t in, int32_t out);
-/* Introspection, host side only (no device work): how the tensor-core kernel deals a projection of this shape to its CTAs.
+/* Introspection, host side only (no device work): how the one-CTA tensor-core kernel deals a projection of this shape to its
+ * CTAs.  (Batches of more than 128 rows whose tiles fill the GPU run on pairs of CTAs instead, with tiles of 256 outputs.)
  * h_plan12 (HOST, 12 int32): [0] token rows per tile, [1] CTAs, [2] row tiles (128 outputs), [3] token tiles, [4] k-blocks
  * (64 of in), [5] k-block steps per CTA, [6] token tiles per group (0: contiguous ranges of k-blocks over all tiles, split
  * tiles handed over between CTAs -- decode sizes), [7] lanes (> 0: CTA c serves token tile c mod [6] of every group and the

@@ -69,7 +69,7 @@ int launch_grouped_tc(const GroupedArgs& ga, void* work, size_t work_bytes, cuda
     case 32: return launch_grouped<32>(ga, work, st);
     case 64: return launch_grouped<64>(ga, work, st);
     case 128: return launch_grouped<128>(ga, work, st);
-    case 256: return launch_grouped<256>(ga, work, st);
+    case 256: return launch_grouped_pair(ga, work, st);
   }
   return fail(MLORA_EINVAL, "grouped_linear: rows per tile must be 16, 32, 64, 128 or 256 (got %d)", ga.tile_rows);
 }

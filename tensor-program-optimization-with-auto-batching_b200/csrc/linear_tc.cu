@@ -90,7 +90,8 @@ Plan plan_for(int bn, int min_waves, int T, int in, int out) {
 
 // 256-token tiles where whole tiles fill the grid at least three times over (prompt passes of thousands of rows): a
 // 128 x 128 tile moves 64 KB through shared memory per 256 tensor-pipe cycles, twice what a shared memory delivers;
-// 128 x 256 moves 96 KB per 512.  Switch: MLORA_TILE256=0 keeps 128-token tiles.
+// 128 x 256 moves 96 KB per 512.  (Calls whose expand runs on CUDA cores; the others of this size go to pairs of CTAs, which
+// are faster: linear_pair_tc.cu.)  Switch: MLORA_TILE256=0 keeps 128-token tiles.
 bool tile256_enabled() {
   static const bool on = [] {
     const char* e = getenv("MLORA_TILE256");
@@ -176,11 +177,13 @@ int launch(const LinearArgs& a, const Plan& pl, void* work, cudaStream_t st) {
   int dev = 0;
   cudaGetDevice(&dev);
   if (!((attr_done.load(std::memory_order_acquire) >> (dev & 63)) & 1ull)) {
-    cudaError_t e = cudaFuncSetAttribute(linear_tc_kernel<BN, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(linear_tc_kernel<BN, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(linear_tc_kernel<BN, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    cudaError_t e = cudaFuncSetAttribute(linear_tc_kernel<BN, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    if constexpr (BN < 256) {
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(linear_tc_kernel<BN, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+      if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(linear_tc_kernel<BN, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::kSmemBytes);
+    }
     if (e != cudaSuccess) return fail(MLORA_ECUDA, "linear: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     attr_done.fetch_or(1ull << (dev & 63), std::memory_order_release);
   }
@@ -204,12 +207,19 @@ int launch(const LinearArgs& a, const Plan& pl, void* work, cudaStream_t st) {
       return MLORA_OK;
     }
   }
-  if (p.lora_mode == 1)
+  if constexpr (BN == 256) {
+    // Everything else of this size runs on pairs of CTAs: enough whole 256-token tiles for this plan are more than enough for
+    // linear_pair_supported(), which leaves only the expand on CUDA cores.
+    if (p.lora_mode != 1) return fail(MLORA_EINVAL, "linear: no one-CTA kernel for 256-token tiles without a CUDA-core expand");
     launch_pdl_if(pdl_enabled_gemm(), linear_tc_kernel<BN, 1>, pl.grid, kThreads, C::kSmemBytes, st, mw, mx, mb, my, p);
-  else if (p.lora_mode == 2 || (a.flags & MLORA_SHARE_LORA_KERNEL))
-    launch_pdl_if(pdl_enabled_gemm(), linear_tc_kernel<BN, 2>, pl.grid, kThreads, C::kSmemBytes, st, mw, mx, mb, my, p);
-  else
-    launch_pdl_if(pdl_enabled_gemm(), linear_tc_kernel<BN, 0>, pl.grid, kThreads, C::kSmemBytes, st, mw, mx, mb, my, p);
+  } else {
+    if (p.lora_mode == 1)
+      launch_pdl_if(pdl_enabled_gemm(), linear_tc_kernel<BN, 1>, pl.grid, kThreads, C::kSmemBytes, st, mw, mx, mb, my, p);
+    else if (p.lora_mode == 2 || (a.flags & MLORA_SHARE_LORA_KERNEL))
+      launch_pdl_if(pdl_enabled_gemm(), linear_tc_kernel<BN, 2>, pl.grid, kThreads, C::kSmemBytes, st, mw, mx, mb, my, p);
+    else
+      launch_pdl_if(pdl_enabled_gemm(), linear_tc_kernel<BN, 0>, pl.grid, kThreads, C::kSmemBytes, st, mw, mx, mb, my, p);
+  }
   count_launch();
   MLORA_CHECK_LAUNCH("linear_tc_kernel");
   return MLORA_OK;
@@ -294,7 +304,7 @@ bool linear_tc_supported(const LinearArgs& a) {
          tiles * ((a.in + BK - 1) / BK) < 2000000000ll;
 }
 
-// How a projection of this shape is dealt to the CTAs (host-side planning only; no device work).
+// How a projection of this shape is dealt to the CTAs of the one-CTA kernel (host-side planning only; no device work).
 void linear_tc_plan(int T, int in, int out, int32_t* v) {
   const Plan pl = make_plan(T, in, out);
   v[0] = pl.bn;
@@ -319,6 +329,7 @@ size_t linear_tc_workspace(int T, int in, int out) {
 int launch_linear_tc(const LinearArgs& a, void* work, size_t work_bytes, cudaStream_t st) {
   const size_t need = linear_tc_workspace(a.T, a.in, a.out);
   if (work_bytes < need) return fail(MLORA_ESIZE, "linear: workspace of %zu bytes needed, %zu given", need, work_bytes);
+  if (linear_pair_supported(a)) return launch_linear_pair(a, work, st);
   Plan pl = make_plan(a.T, a.in, a.out);
   switch (pl.bn) {
     case 16: return launch<16>(a, pl, work, st);

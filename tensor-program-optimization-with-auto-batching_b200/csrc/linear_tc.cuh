@@ -13,7 +13,7 @@
 //   * decode sizes (stream-K): the iteration space (tile, k-block) -- tiles = row tiles x token tiles,
 //     k-blocks of 64 -- is cut into equal contiguous ranges, one per CTA, so every SM streams the same
 //     number of bytes whatever the shape; a range covers a tail of one tile, whole tiles, and a head of
-//     another.  Prefill sizes: whole tiles of 128 or 256 tokens only, dealt in token-tile groups whose CTAs walk
+//     another.  Prefill sizes that do not go to pairs of CTAs (linear_pair_tc.cu): whole tiles of 128 or 256 tokens only, dealt in token-tile groups whose CTAs walk
 //     the row tiles in lockstep lanes (see wave_tile);
 //   * two TMEM accumulators: the epilogue of one segment overlaps the MMAs of the next, and the
 //     shared-memory ring keeps filling across segment boundaries;
@@ -80,31 +80,33 @@ struct TcParams {
   float* partials;  // [grid][2][BN][BM]
 };
 
-// Distinct adapter slots among the tokens of one token tile, in order of first appearance.
-// Executed by one full warp; s_tok [BN] receives the tile's slots, s_list [BN] the distinct ones.
-template <int BN>
-__device__ __forceinline__ int distinct_slots(const LinearArgs& a, int t0, int* s_tok, int* s_list) {
+// Distinct adapter slots among the first `rows` tokens from t0, in order of first appearance.
+// Executed by one full warp; s_tok [n_tok] receives the tile's slots, s_list [n_tok] the distinct ones.
+__device__ __forceinline__ int distinct_slots_n(const LinearArgs& a, int t0, int rows, int n_tok, int* s_tok, int* s_list) {
   const int lane = threadIdx.x & 31;
-  for (int n = lane; n < BN; n += 32) {
-    int s = (t0 + n < a.T) ? a.slots[t0 + n] : -1;
-    s_tok[n] = (s >= 0 && s < a.n_adapters) ? s : -1;
-  }
-  __syncwarp();
   int count = 0;
 #pragma unroll 1
-  for (int base = 0; base < BN; base += 32) {
+  for (int base = 0; base < n_tok; base += 32) {
     const int n = base + lane;
-    const int s = n < BN ? s_tok[n] : -1;
-    bool first = s >= 0;
-    for (int m = 0; first && m < n; ++m) first = s_tok[m] != s;
+    int s = n < rows && n < n_tok ? a.slots[t0 + n] : -1;
+    if (s >= a.n_adapters || s < 0) s = -1;
+    if (n < n_tok) s_tok[n] = s;
+    // the first of its adapter among these 32 (every lane takes part), and not listed yet
+    const unsigned same = __match_any_sync(0xffffffffu, s);
+    bool first = s >= 0 && (same & ((1u << lane) - 1)) == 0;
+#pragma unroll 4
+    for (int m = 0; m < count; ++m) first &= s_list[m] != s;
     const unsigned mask = __ballot_sync(0xffffffffu, first);
     if (first) s_list[count + __popc(mask & ((1u << lane) - 1))] = s;
     count += __popc(mask);
+    __syncwarp();
   }
-  __syncwarp();
   return count;
 }
-
+template <int BN>
+__device__ __forceinline__ int distinct_slots(const LinearArgs& a, int t0, int* s_tok, int* s_list) {
+  return distinct_slots_n(a, t0, a.T - t0, BN, s_tok, s_list);
+}
 
 // Four adjacent outputs of one token: one 8-byte (bf16) or 16-byte (fp32) store when aligned and
 // all four exist, scalar stores otherwise.
@@ -208,16 +210,15 @@ __device__ __forceinline__ bool lora_cached(const TcParams& p, int n_seg) {
 // BN + 16 rows per adapter at most, whatever the number of adapters.  Returns the total number of operand rows, or -1 when
 // some adapter's rows are scattered (or there are more than 16 adapters).  One full warp; s_tok / s_list as written by
 // distinct_slots; tab (optional, [16]): per adapter (first accumulator column, rows, row offset of its operand).
-template <int BN>
-__device__ __forceinline__ int adapter_runs(const int* s_tok, const int* s_list, int n_seg, int4* tab) {
-  if (BN < 128 || n_seg > 16) return -1;
+__device__ __forceinline__ int adapter_runs_n(int n_tok, const int* s_tok, const int* s_list, int n_seg, int4* tab) {
+  if (n_seg > 16) return -1;
   const int lane = threadIdx.x & 31;
   int total = 0;
   bool ok = true;
   for (int j = 0; j < n_seg; ++j) {
     const int s = s_list[j];
-    int lo = BN, hi = -1, cnt = 0;
-    for (int r = lane; r < BN; r += 32)
+    int lo = n_tok, hi = -1, cnt = 0;
+    for (int r = lane; r < n_tok; r += 32)
       if (s_tok[r] == s) {
         lo = min(lo, r);
         hi = max(hi, r);
@@ -232,6 +233,10 @@ __device__ __forceinline__ int adapter_runs(const int* s_tok, const int* s_list,
     total += rows;
   }
   return ok ? total : -1;
+}
+template <int BN>
+__device__ __forceinline__ int adapter_runs(const int* s_tok, const int* s_list, int n_seg, int4* tab) {
+  return BN < 128 ? -1 : adapter_runs_n(BN, s_tok, s_list, n_seg, tab);
 }
 // Operands of a tile in the shared-memory cache: in the run layout when the rows allow it and it fits, else as full-height
 // masked operands per adapter when those fit.
@@ -288,13 +293,13 @@ __device__ __forceinline__ int wave_tile(const TcParams& p, int lt) {
   const int j = q / p.row_tiles;
   return (group * p.wave_gt + j) * p.row_tiles + (q - j * p.row_tiles);
 }
-__device__ __forceinline__ GroupTile group_tile(const TcParams& p, int tok_tile, int bn) {
-  if (p.g.table != nullptr) {
-    const int4 e = __ldg(reinterpret_cast<const int4*>(p.g.table) + 1 + tok_tile);
+__device__ __forceinline__ GroupTile group_tile(const Groups& g, int T, int tok_tile, int bn) {
+  if (g.table != nullptr) {
+    const int4 e = __ldg(reinterpret_cast<const int4*>(g.table) + 1 + tok_tile);
     return GroupTile{e.x, e.y, e.z};
   }
-  const int grp = tok_tile / p.g.tiles_per_group, row0 = (tok_tile - grp * p.g.tiles_per_group) * bn;
-  return GroupTile{grp, row0, min(bn, p.a.T - row0)};
+  const int grp = tok_tile / g.tiles_per_group, row0 = (tok_tile - grp * g.tiles_per_group) * bn;
+  return GroupTile{grp, row0, min(bn, T - row0)};
 }
 // GRP: the number of tiles may be known on the device only.  Token tiles below 128 rows: equal k-block ranges over all
 // tiles as for a plain decode-size projection; larger ones: whole tiles, dealt round robin (neighbouring CTAs then share
@@ -512,7 +517,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc_kernel(const __grid_con
       if (WAVE && sg.tile < 0) break;
       const int row_tile = sg.tile % p.row_tiles, tok_tile = sg.tile / p.row_tiles;
       if (lane == 0) {
-        if constexpr (GRP) wp = reinterpret_cast<const uint8_t*>(a.W) + (size_t)group_tile(p, tok_tile, BN).group * p.g.w_bytes;
+        if constexpr (GRP) wp = reinterpret_cast<const uint8_t*>(a.W) + (size_t)group_tile(p.g, p.a.T, tok_tile, BN).group * p.g.w_bytes;
         int nn = n;
         for (int kb = sg.kb0; kb < sg.kb1; ++kb, ++nn) {
           const int s = nn % C::kWStages, round = nn / C::kWStages;
@@ -594,7 +599,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc_kernel(const __grid_con
       if (WAVE && sg.tile < 0) break;
       const int row_tile = sg.tile % p.row_tiles, tok_tile = sg.tile / p.row_tiles;
       if constexpr (GRP) {
-        const GroupTile gt = group_tile(p, tok_tile, BN);
+        const GroupTile gt = group_tile(p.g, p.a.T, tok_tile, BN);
         const int x_col = gt.group * p.g.x_cols;
         // rows gathered four by four; rows past the tile's last repeat it (their outputs are not stored)
         constexpr int kQuads = BN / 4, kPerLane = (kQuads + 31) / 32;
@@ -1000,7 +1005,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc_kernel(const __grid_con
       const int row = row_tile * BM + etid;
       int t0 = tok_tile * BN, t_end = a.T, y_col = 0, group = 0;
       if constexpr (GRP) {
-        const GroupTile gt = group_tile(p, tok_tile, BN);
+        const GroupTile gt = group_tile(p.g, p.a.T, tok_tile, BN);
         t0 = gt.row0;
         t_end = gt.row0 + gt.rows;
         group = gt.group;
