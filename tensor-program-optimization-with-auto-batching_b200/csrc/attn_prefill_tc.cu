@@ -5,16 +5,21 @@
 // One CTA = one tile of up to 128 consecutive prompt rows of ONE sequence x one head.  Per block of 128 keys:
 //   S = Q K^T      tcgen05.mma, M = 128 queries, N = 128 keys, K = head_dim 128; Q and K both K-major in 128-byte-swizzled
 //                  shared memory -- Q by one TMA load per tile, K by one TMA load per page (16 keys) through the block table;
-//   softmax        one thread per query row (= TMEM lane): scores read back with tcgen05.ld, causal mask, online maximum
-//                  and sum, probabilities written as bf16 into the A-operand layout;
-//   O_blk = P V    M = 128 queries, N = 128 head dims, K = 128 keys; V arrives by TMA exactly as the pages hold it,
-//                  [key][dim], and is used as an MN-major B operand (the dimension is the contiguous one): no transpose;
-//                  P is written over the K block, which S = Q K^T has consumed by then;
-//   O = O * exp2(m_old - m_new) + O_blk    in registers (128 fp32 per thread), no read-modify-write of TMEM.
-// Inside a CTA the two MMAs of a block and the softmax between them run one after the other; two CTAs share an SM
-// (96 KB of shared memory and 256 TMEM columns each) and fill each other's gaps.  The point of this kernel is to take
-// prompt attention off the CUDA cores -- the single-query kernel it replaces re-reads every key for every row and
-// reduces every score with shuffles.  Every wait is bounded; a CTA that gives up writes zeros.
+//   softmax        one thread per query row (= TMEM lane): its 128 scores in registers by tcgen05.ld, causal mask, online
+//                  maximum and sum, probabilities as bf16 back into TMEM over the scores;
+//   O += P V       A = P from TMEM, N = 128 head dims, K = 128 keys; V arrives by TMA exactly as the pages hold it,
+//                  [key][dim], and is used as an MN-major B operand (the dimension is the contiguous one): no transpose.
+// O stays in TMEM.  A row's scores are taken relative to a reference that follows its maximum only when that has grown by
+// more than 2^8 (the sum and O share the reference, so the quotient is the same; fp32 has the room, and bf16 probabilities
+// are relative): after the first blocks hardly any row rescales its 128 outputs.
+//
+// What bounds it: the softmax -- 16384 exponentials per block are 1024 cycles of an SM, the two MMAs are 1024 cycles of
+// tensor pipe -- and the chain S -> softmax -> P V of a CTA.  Two CTAs share an SM (96 KB of shared memory and 256 TMEM
+// columns each) and fill each other's gaps; a CTA's own copies are off the chain: K of the next block is fetched from the
+// moment S = Q K^T has read it, V from the moment P V has.  CTAs of late tiles (most keys) start first.
+// Measured (32 heads of 128, keys and values dense, CUDA events), one buffer of K / V and O in registers -> this:
+// 2 x 4096 rows 590 -> 354 us (777 TFLOP/s), 16 x 512 148 -> 104, 64 x 128 97 -> 74, 1 x 8192 1085 -> 639 (860).
+// Every wait is bounded; a CTA that gives up writes zeros.
 #include <math.h>
 
 #include <atomic>
@@ -53,6 +58,7 @@ struct PfArgs {
   int page_parts;   // paged form: page size in 16s
   int chunk;        // > 0: a row sees only positions of its own chunk of this many (counted from position 0)
   const float* sink;  // [Hq] or NULL: a logit per head that only enters the softmax's sum
+  int n_tiles;
 };
 
 // NK, NV: query/key and value size of a head in 64s.  PAGED: keys and values come 16 at a time through the block table,
@@ -66,14 +72,16 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sq = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
   uint8_t* sk = sq + NK * kSub;  // K block   [128 keys][128 d]   as two d-halves
-  uint8_t* sv = sk + 2 * kSub;   // V block   [128 keys][128 d]   as two d-halves, exactly as the pages hold it
-  uint8_t* sp = sk;              // P block   [128 q][128 keys]   as two key-halves: over K, which S = Q K^T has consumed by then
-  __shared__ uint64_t kbar, sbar, obar;
+  uint8_t* sv = sk + NK * kSub;  // V block   [128 keys][128 d]   as two d-halves, exactly as the pages hold it
+  __shared__ uint64_t kbar, vbar;  // a block's K (the first: and Q) / V has landed
+  __shared__ uint64_t sbar;        // S = Q K^T has retired, and every P V before it
+  __shared__ uint64_t pbar;        // the four softmax warps have written P (and rescaled O)
+  __shared__ uint64_t obar, dbar;  // P V has retired / the last one has
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int tile = blockIdx.x, h = blockIdx.y;
+  const int tile = a.n_tiles - 1 - (int)(blockIdx.x / a.Hq), h = blockIdx.x % a.Hq;
   const int rep = a.Hq / a.Hkv, kvh = h / rep;
   const int slot = a.tiles[tile * 4 + 0], row0 = a.tiles[tile * 4 + 1], rows = a.tiles[tile * 4 + 2], pos0 = a.tiles[tile * 4 + 3];
   const int32_t* bt = PAGED ? a.block_table + (size_t)slot * a.max_pages : nullptr;
@@ -88,8 +96,11 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
   if (tid == 0) {
     s_abort = 0;
     mbar_init(&kbar, 1);
+    mbar_init(&vbar, 1);
     mbar_init(&sbar, 1);
+    mbar_init(&pbar, 4);
     mbar_init(&obar, 1);
+    mbar_init(&dbar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_k);
@@ -99,77 +110,50 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = tmem_slot;
-  constexpr uint32_t idesc = make_idesc(kTile, kTile);
-  constexpr uint32_t idesc_pv = make_idesc(kTile, kDv) | (1u << 16);  // B operand MN-major
+  const uint32_t tmem_base = tmem_slot, tmem_o = tmem_base + kTile;
 
-  // per-row state (threads 0..127)
-  float o_reg[kDv];
-#pragma unroll
-  for (int i = 0; i < kDv; ++i) o_reg[i] = 0.f;
-  const int q_pos = pos0 + tid;  // position of this thread's query row
-  const int q_lo = q_pos - q_pos % chunk;  // first key it sees
-  const float scale = a.scale * kLog2e;
-  float m_run = a.sink ? a.sink[h] * kLog2e : -INFINITY, l_run = a.sink ? 1.f : 0.f;
-  bool ok = true;
-
-  // Block-table entries are read one block ahead (lane p of warp 4 keeps page p of the block's eight), so that no block
-  // starts with a dependent chain of two global round trips.
-  // (row of the first of 16 keys in the pages seen as rows; a missing entry reads as rows before 0: zeros)
-  auto page_of = [&](int pg) {
-    return pg < n_pages ? ((bt[pg / a.page_parts] * a.Hkv + kvh) * a.page_parts + pg % a.page_parts) * kPS : -kPS;
-  };
-  int page_next = (PAGED && warp == 4 && lane < kTile / kPS) ? page_of(key0 / kPS + lane) : -kPS;
-
-  for (int kb = 0; kb < n_blocks; ++kb) {
-    const uint32_t par = kb & 1;
-    const int kstart = key0 + kb * kTile;  // first key of the block
-    const int page0 = kstart / kPS;
-    const int page_cur = page_next;
-    const int valid = min(kTile / kPS, n_pages - page0);
-    if (PAGED && kb + 1 < n_blocks && warp == 4 && lane < kTile / kPS) page_next = page_of(page0 + kTile / kPS + lane);
-    // ---- loads: K and V pages (and Q once) by TMA -----------------------------------------------------------------------------
-    if (warp == 4) {
+  if (warp == 4) {
+    // ---- copies and MMAs: lane 0 waits and issues, eight lanes copy a page each -----------------------------------------
+    constexpr uint32_t idesc = make_idesc(kTile, kTile);
+    constexpr uint32_t idesc_pv = make_idesc(kTile, kDv) | (1u << 16);  // B operand MN-major
+    auto wait = [&](uint64_t* bar, uint32_t par) {
+      int w = 1;
+      if (lane == 0) w = mbar_wait(bar, par, &s_abort) ? 1 : 0;
+      w = __shfl_sync(0xffffffffu, w, 0);
+      if (!w) s_abort = 1;
+      return w != 0;
+    };
+    // Block-table entries are read one block ahead (lane p keeps page p of the block's eight), so that no block starts with
+    // a dependent chain of two global round trips.
+    // (row of the first of 16 keys in the pages seen as rows)
+    auto page_of = [&](int kb) {
+      const int pg = key0 / kPS + kb * (kTile / kPS) + lane;
+      return PAGED && lane < kTile / kPS && pg < n_pages
+                 ? ((bt[pg / a.page_parts] * a.Hkv + kvh) * a.page_parts + pg % a.page_parts) * kPS : -kPS;
+    };
+    auto copy = [&](int kb, int page, uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int parts, int col, uint32_t more) {
+      const int valid = PAGED ? min(kTile / kPS, n_pages - key0 / kPS - kb * (kTile / kPS)) : 0;
       if (lane == 0) {
-        mbar_expect_tx(&kbar, (PAGED ? (uint32_t)valid * (NK + NV) * (kPS * 128) : (uint32_t)(NK + NV) * kSub) + (kb == 0 ? NK * kSub : 0));
-        if (kb == 0) {
-#pragma unroll
-          for (int j = 0; j < NK; ++j) tma_load_2d(sq + j * kSub, &map_q, h * NK * 64 + j * 64, row0, &kbar);
-        }
-        if constexpr (!PAGED) {  // rows past the sequence's last key belong to the next one (or are zeros): masked
-#pragma unroll
-          for (int j = 0; j < NK; ++j) tma_load_2d(sk + j * kSub, &map_k, h * NK * 64 + j * 64, slot + kb * kTile, &kbar);
-#pragma unroll
-          for (int j = 0; j < NV; ++j)
-            tma_load_2d(sv + j * kSub, &map_v, a.v_col + h * NV * 64 + j * 64, slot + kb * kTile, &kbar);
-        }
+        mbar_expect_tx(bar, (PAGED ? (uint32_t)(valid * parts * kPS * 128) : (uint32_t)(parts * kSub)) + more);
+        if constexpr (!PAGED)  // rows past the sequence's last key belong to the next one (or are zeros): masked
+          for (int j = 0; j < parts; ++j) tma_load_2d(dst + j * kSub, map, col + j * 64, slot + kb * kTile, bar);
       }
       __syncwarp();
-      if (PAGED && lane < valid) {  // 16 keys per lane, every 64-column part of K and of V
-#pragma unroll
-        for (int j = 0; j < NK; ++j) tma_load_2d(sk + j * kSub + lane * (kPS * 128), &map_k, j * 64, page_cur, &kbar);
-#pragma unroll
-        for (int j = 0; j < NV; ++j) tma_load_2d(sv + j * kSub + lane * (kPS * 128), &map_v, j * 64, page_cur, &kbar);
-      }
-    } else if (n_keys - kstart < kTile) {
-      // Last block, not full: the V rows of keys that do not exist (the tail of the last page, whatever the cache holds
-      // there, and the pages that were not loaded) are zeroed once the copies have landed -- their probabilities are 0,
-      // but 0 * NaN is not.  K needs nothing: those scores are masked.  (A swizzled row stays inside its own 128 bytes.)
-      if (!mbar_wait(&kbar, par, &s_abort)) s_abort = 1;
-      if (tid >= n_keys - kstart) {
-#pragma unroll
-        for (int half = 0; half < NV; ++half)
-#pragma unroll
-          for (int c = 0; c < 8; ++c) reinterpret_cast<uint4*>(sv + half * kSub + tid * 128)[c] = make_uint4(0u, 0u, 0u, 0u);
-      }
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    // ---- S = Q K^T ----------------------------------------------------------------------------------------------------------
-    if (tid == 128) {
-      if (!mbar_wait(&kbar, par, &s_abort)) s_abort = 1;
-      tc_fence_after();
-      if (!s_abort) {
+      if (PAGED && lane < valid)  // 16 keys per lane, every 64-column part
+        for (int j = 0; j < parts; ++j) tma_load_2d(dst + j * kSub + lane * (kPS * 128), map, j * 64, page, bar);
+      __syncwarp();
+    };
+    const int k_col = h * NK * 64, v_col = a.v_col + h * NV * 64;
+    int page = page_of(0), page_next = page_of(1);
+    copy(0, page, sk, &map_k, &kbar, NK, k_col, NK * kSub);
+    if (lane == 0)
+      for (int j = 0; j < NK; ++j) tma_load_2d(sq + j * kSub, &map_q, k_col + j * 64, row0, &kbar);
+    copy(0, page, sv, &map_v, &vbar, NV, v_col, 0);
+    for (int kb = 0; kb < n_blocks; ++kb) {
+      const uint32_t par = kb & 1;
+      if (!wait(&kbar, par)) break;
+      if (lane == 0) {
+        tc_fence_after();
 #pragma unroll
         for (int j = 0; j < NK; ++j) {
           const uint64_t adesc = make_smem_desc(smem_u32(sq + j * kSub));
@@ -177,141 +161,154 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
 #pragma unroll
           for (int k = 0; k < 4; ++k) umma_bf16(tmem_base, adesc + 2 * k, bdesc + 2 * k, idesc, (j > 0 || k > 0) ? 1u : 0u);
         }
+        umma_commit(&sbar);
       }
-      umma_commit(&sbar);
+      if (kb > 0) {  // V's place is free once the P V before has retired (as it has when this S retires)
+        if (!wait(&obar, par ^ 1)) break;
+        copy(kb, page, sv, &map_v, &vbar, NV, v_col, 0);
+      }
+      if (kb + 1 < n_blocks) {
+        if (!wait(&sbar, par)) break;
+        page = page_next;
+        page_next = page_of(kb + 2);
+        copy(kb + 1, page, sk, &map_k, &kbar, NK, k_col, 0);
+      }
+      if (!wait(&vbar, par) || !wait(&pbar, par)) break;
+      if (lane == 0) {
+        tc_fence_after();
+        // A = P in TMEM, two keys per column: 16 keys are 8 columns.  B = V as the pages hold it, [key][dim]: the dimension
+        // (N) is the contiguous one ("MN-major"), 64 of it per 128-byte row, the second 64 one sub-tile (leading byte
+        // offset) further, 8 keys per 1024-byte swizzle group (stride byte offset), 16 keys = 2048 bytes.
+#pragma unroll
+        for (int k = 0; k < kTile / 16; ++k)
+          umma_bf16_ta(tmem_o, tmem_base + k * 8, make_smem_desc_mn(smem_u32(sv + k * 2048), kSub, 1024), idesc_pv,
+                       (kb > 0 || k > 0) ? 1u : 0u);
+        umma_commit(&obar);
+        if (kb + 1 == n_blocks) umma_commit(&dbar);
+      }
+      __syncwarp();
     }
-    float corr = 1.f;
-    if (tid < kTile) {
-      if (!mbar_wait(&sbar, par, &s_abort)) s_abort = 1;
+    if (s_abort && lane == 0)  // copies may still be in flight: let them land before the shared memory goes to another CTA
+      for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  } else {
+    // ---- softmax: one thread per query row --------------------------------------------------------------------------------
+    const int q_pos = pos0 + tid;  // position of this thread's query row
+    const int q_lo = q_pos - q_pos % chunk;  // first key it sees
+    const float scale = a.scale * kLog2e;
+    const uint32_t lanes = (uint32_t)(warp * 32) << 16;
+    // reference of the row's scores, and their sum relative to it (a sink: a score of its own without a value)
+    float m_ref = a.sink ? a.sink[h] * kLog2e : -INFINITY, l_run = a.sink ? 1.f : 0.f;
+    bool ok = true;
+    for (int kb = 0; kb < n_blocks && ok; ++kb) {
+      const uint32_t par = kb & 1;
+      const int kstart = key0 + kb * kTile;  // first key of the block
+      ok = __all_sync(0xffffffffu, mbar_wait(&sbar, par, &s_abort));
+      if (!ok) break;
       tc_fence_after();
-      const uint32_t t_addr = tmem_base + ((uint32_t)(warp * 32) << 16);
+      float s[kTile];
+#pragma unroll
+      for (int c0 = 0; c0 < kTile; c0 += 32) tmem_ld32_issue(tmem_base + lanes + c0, s + c0);
+      tmem_wait_ld();
       // Only the blocks on or past the diagonal need the causal / length mask, and those before the last row's chunk the
       // chunk's (uniform per CTA): every row of the tile sees every key of the blocks between.
       const bool need_mask = kstart + kTile - 1 > pos0 || kstart < lo_last;
-      // pass 1: row maximum over the valid keys (of the raw scores: the scale is positive)
-      float mx = -INFINITY;
+      if (need_mask) {
+        const int hi = min(q_pos, n_keys - 1) - kstart, lo = q_lo - kstart;
+#pragma unroll
+        for (int i = 0; i < kTile; ++i)
+          if (i > hi || i < lo) s[i] = -INFINITY;
+      }
+      // row maximum (of the raw scores: the scale is positive)
+      float mx[4] = {s[0], s[1], s[2], s[3]};
+#pragma unroll
+      for (int i = 4; i < kTile; ++i) mx[i & 3] = fmaxf(mx[i & 3], s[i]);
+      const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale;
+      // a new reference: at the first visible key, and when the maximum has outgrown the old one
+      const bool grow = kb == 0 ? m_blk > m_ref : m_blk > m_ref + 8.f;
+      if (__any_sync(0xffffffffu, grow)) {
+        const float corr = grow ? (m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - m_blk)) : 1.f;
+        if (grow) m_ref = m_blk;
+        l_run *= corr;
+        if (kb > 0) {  // (every P V so far has retired: sbar)
 #pragma unroll 1
-      for (int c0 = 0; c0 < kTile; c0 += 32) {
-        float s[32];
-        tmem_ld32(t_addr + c0, s);
-        if (!need_mask) {
+          for (int c0 = 0; c0 < kDv; c0 += 32) {
+            float o[32];
+            tmem_ld32(tmem_o + lanes + c0, o);
 #pragma unroll
-          for (int i = 0; i < 32; ++i) mx = fmaxf(mx, s[i]);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int key = kstart + c0 + i;
-            if (key <= q_pos && key >= q_lo && key < n_keys) mx = fmaxf(mx, s[i]);
+            for (int i = 0; i < 32; ++i) o[i] *= corr;
+            tmem_st<32>(tmem_o + lanes + c0, o);
           }
         }
       }
-      const float m_new = fmaxf(m_run, mx * scale);
-      corr = (m_run == -INFINITY) ? 0.f : fast_exp2(m_run - m_new);  // (m_new == -inf: nothing seen yet, l and o are 0 anyway)
-      const float neg_m = m_new == -INFINITY ? 0.f : -m_new;       // (then every key of the block is masked)
-      // pass 2: probabilities -> P (bf16, A-operand layout), row sum
-      float lsum = 0.f;
-#pragma unroll 1
-      for (int c0 = 0; c0 < kTile; c0 += 32) {
-        float s[32];
-        tmem_ld32(t_addr + c0, s);
+      const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref;  // (then every key so far is masked: probabilities are 0)
+      // probabilities -> P (bf16 pairs), row sum
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-          float p[8];
-          if (!need_mask) {
+      for (int c0 = 0; c0 < kTile; c0 += 64) {
+        float pk[32];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              p[i] = fast_exp2(fmaf(s[g * 8 + i], scale, neg_m));
-              lsum += p[i];
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int key = kstart + c0 + g * 8 + i;
-              const bool valid = key <= q_pos && key >= q_lo && key < n_keys;
-              p[i] = valid ? fast_exp2(fmaf(s[g * 8 + i], scale, neg_m)) : 0.f;
-              lsum += p[i];
-            }
-          }
-          const int keyc = c0 + g * 8;  // first key of this 16-byte chunk inside the block
-          const int cx = (keyc & 63) >> 3;
-          *reinterpret_cast<uint4*>(sp + (keyc >> 6) * kSub + tid * 128 + ((cx ^ (tid & 7)) << 4)) = pack8(p);
+        for (int i = 0; i < 32; ++i) {
+          const float p0 = fast_exp2(fmaf(s[c0 + 2 * i], scale, neg_m)), p1 = fast_exp2(fmaf(s[c0 + 2 * i + 1], scale, neg_m));
+          sum[(2 * i) & 3] += p0;
+          sum[(2 * i + 1) & 3] += p1;
+          const __nv_bfloat162 b = __floats2bfloat162_rn(p0, p1);
+          pk[i] = __uint_as_float(*reinterpret_cast<const uint32_t*>(&b));
         }
+        tmem_st<32>(tmem_base + lanes + c0 / 2, pk);
       }
-      l_run = l_run * corr + lsum;
-      m_run = m_new;
-      tc_fence_before();
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    // ---- O_blk = P V ----------------------------------------------------------------------------------------------------------
-    if (tid == 128) {
-      tc_fence_after();
-      if (!s_abort) {
+      l_run += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+      if (n_keys - kstart < kTile) {
+        // Last block, not full: the V rows of keys that do not exist (the tail of the last page, whatever the cache holds
+        // there, and the pages that were not loaded) are zeroed once the copies have landed -- their probabilities are 0,
+        // but 0 * NaN is not.  K needs nothing: those scores are masked.  (A swizzled row stays inside its own 128 bytes.)
+        ok = __all_sync(0xffffffffu, mbar_wait(&vbar, par, &s_abort));
+        if (!ok) break;
+        if (tid >= n_keys - kstart) {
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          // A = P, K-major: 16 keys further = 32 bytes = +2 in the address field.  B = V as the pages hold it, [key][dim]:
-          // the dimension (N) is the contiguous one ("MN-major"), 64 of it per 128-byte row, the second 64 one sub-tile
-          // (leading byte offset) further, 8 keys per 1024-byte swizzle group (stride byte offset), 16 keys = 2048 bytes.
-          const uint64_t adesc = make_smem_desc(smem_u32(sp + j * kSub));
+          for (int half = 0; half < NV; ++half)
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            umma_bf16(tmem_base + kTile, adesc + 2 * k, make_smem_desc_mn(smem_u32(sv + (j * 4 + k) * 2048), kSub, 1024), idesc_pv,
-                      (j > 0 || k > 0) ? 1u : 0u);
+            for (int c = 0; c < 8; ++c) reinterpret_cast<uint4*>(sv + half * kSub + tid * 128)[c] = make_uint4(0u, 0u, 0u, 0u);
         }
-      }
-      umma_commit(&obar);
-      // the next block's K loads and MMAs reuse sk / sp / TMEM: wait here until this block's MMAs have retired
-      if (!mbar_wait(&obar, par, &s_abort)) s_abort = 1;
-    }
-    if (tid < kTile) {
-      if (!mbar_wait(&obar, par, &s_abort)) s_abort = 1;
-      tc_fence_after();
-      const uint32_t t_addr = tmem_base + ((uint32_t)(warp * 32) << 16) + kTile;
-#pragma unroll
-      for (int c0 = 0; c0 < kDv; c0 += 32) {
-        float blk[32];
-        tmem_ld32(t_addr + c0, blk);
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o_reg[c0 + i] = fmaf(o_reg[c0 + i], corr, blk[i]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       }
       tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&pbar);
     }
-    __syncthreads();  // sv / sp / TMEM free for the next block; s_abort settled
-    if (s_abort) {
-      ok = false;
-      // a wait expired: before the CTA leaves (and its shared memory goes to another CTA) give this block's copies,
-      // which may still be in flight, one more bounded wait to land
-      if (tid == 128) {
-        int none = 0;
-        mbar_wait(&kbar, par, &none);
-      }
-      break;
-    }
-  }
-
-  // ---- write ------------------------------------------------------------------------------------------------------------------
-  if (tid < kTile && tid < rows) {
+    ok = ok && __all_sync(0xffffffffu, mbar_wait(&dbar, 0, &s_abort));
+    if (!ok) s_abort = 1;
+    tc_fence_after();
+    // ---- write ----------------------------------------------------------------------------------------------------------
     float inv = (ok && l_run > 0.f) ? 1.f / l_run : 0.f;
     if constexpr (!PAGED)
-      if (a.gate) inv /= 1.f + __expf(-__bfloat162float(a.gate[(size_t)(row0 + tid) * a.ld_gate + h]));
+      if (a.gate && tid < rows) inv /= 1.f + __expf(-__bfloat162float(a.gate[(size_t)(row0 + tid) * a.ld_gate + h]));
     uint4* dst = reinterpret_cast<uint4*>(a.out + (size_t)(row0 + tid) * a.ld_out + (size_t)h * kDv);
 #pragma unroll
-    for (int c = 0; c < kDv / 8; ++c) {
-      float f[8];
+    for (int c0 = 0; c0 < kDv; c0 += 32) {
+      float o[32];
+      tmem_ld32(tmem_o + lanes + c0, o);
+      if (tid < rows) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) f[i] = o_reg[c * 8 + i] * inv;
-      dst[c] = pack8(f);
+        for (int c = 0; c < 4; ++c) {
+          float f[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) f[i] = ok ? o[c * 8 + i] * inv : 0.f;
+          dst[c0 / 8 + c] = pack8(f);
+        }
+      }
     }
+    if (!ok && tid == 0 && a.status) atomicOr(a.status, 1);
   }
-  if (!ok && tid == 0 && a.status) atomicOr(a.status, 1);
   tc_fence_before();
   __syncthreads();
   if (warp == 4) tmem_dealloc(tmem_base, 256);
 }
 
 template <int NK, int NV, bool PAGED>
-int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const PfArgs& a, int n_tiles, cudaStream_t st) {
-  constexpr int smem = (NK + 2 + NV) * kSub + 1024;  // Q, K (= P), V
+int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, PfArgs a, int n_tiles, cudaStream_t st) {
+  if ((long long)n_tiles * a.Hq > 2147483647ll) return fail(MLORA_ESIZE, "prefill_attention: too many tiles x heads");
+  a.n_tiles = n_tiles;
+  constexpr int smem = (2 * NK + NV) * kSub + 1024;  // Q, K, V
   static std::atomic<unsigned long long> attr_done{0};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -320,7 +317,7 @@ int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorM
     if (e != cudaSuccess) return fail(MLORA_ECUDA, "prefill_attention: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     attr_done.fetch_or(1ull << (dev & 63), std::memory_order_release);
   }
-  prefill_attn_tc_kernel<NK, NV, PAGED><<<dim3(n_tiles, a.Hq), kPfThreads, smem, st>>>(mq, mk, mv, a);
+  prefill_attn_tc_kernel<NK, NV, PAGED><<<(unsigned)((long long)n_tiles * a.Hq), kPfThreads, smem, st>>>(mq, mk, mv, a);
   count_launch();
   MLORA_CHECK_LAUNCH("prefill_attn_tc_kernel");
   return MLORA_OK;

@@ -1,6 +1,6 @@
 """Projections of prompt-size batches on pairs of CTAs, at the edges of their tiles, against fp32 torch on the same values.
 
-Both sides sum in fp32 and round once to bf16 (2^-9 of a value at most), so 2^-8 of the result's norm bounds their distance;
+Sums are fp32 and the result is rounded once to bf16 (8 significant bits), so 2^-8 of the result's norm bounds the distance;
 fp32 outputs differ by the order of the sums only.
 """
 import pytest
