@@ -7,11 +7,23 @@ per sequence, ``capture_decode`` / :class:`DecodeSession` the same as a CUDA gra
 """
 from __future__ import annotations
 
+import struct
+
 import numpy as np
 import torch
 
 from . import ops
 from .kv_cache import PagedCache
+
+
+def _int32(tokens):
+    """Token ids as an int32 array (a list of thousands of ids is packed in half the time numpy takes to look at it)."""
+    if type(tokens) is list:
+        try:
+            return np.frombuffer(struct.pack(f"{len(tokens)}i", *tokens), dtype=np.int32)
+        except struct.error:  # not plain 32-bit ids: numpy converts or refuses them
+            pass
+    return np.asarray(tokens, dtype=np.int32)
 
 
 class EngineBase:
@@ -69,6 +81,15 @@ class EngineBase:
         t = torch.as_tensor(np.asarray(values), dtype=dtype)
         dst[: t.numel()].copy_(t.pin_memory(), non_blocking=True)
 
+    def _stage_all(self, *parts):
+        """Copies int32 arrays to the starts of device buffers: (buffer, array) pairs, through one pinned buffer."""
+        parts = [(dst, np.asarray(v, dtype=np.int32).reshape(-1)) for dst, v in parts]
+        pinned = torch.from_numpy(np.concatenate([v for _, v in parts])).pin_memory()
+        a = 0
+        for dst, v in parts:
+            dst[:v.size].copy_(pinned[a:a + v.size], non_blocking=True)
+            a += v.size
+
     def extend(self, seq_ids, portions, adapter_slots=None, want=None, use_lora=True):
         """Runs the next tokens (``portions``: lists of token ids) of already-added sequences from wherever each stands,
         cut into passes of at most ``max_rows`` rows.  ``want[i]``: places inside portion i whose logits are asked for
@@ -100,19 +121,15 @@ class EngineBase:
                     nxt.append((i, start + n))
             pending = nxt
             T = sum(n for _, _, n in chunk)
-            toks = np.concatenate([np.asarray(portions[i][s:s + n], dtype=np.int32) for i, s, n in chunk])
-            slots = np.concatenate([np.full(n, adapter_slots[i], dtype=np.int32) for i, _, n in chunk])
+            lens = [n for _, _, n in chunk]
+            toks = np.concatenate([_int32(portions[i] if n == len(portions[i]) else portions[i][s:s + n]) for i, s, n in chunk])
             passes, a = [], 0
             for i, _, n in chunk:
                 passes.append((seq_ids[i], a, n, kv.length(seq_ids[i])))
                 a += n
-            row_slot, row_pos = kv.begin_forward([seq_ids[i] for i, _, _ in chunk], [n for _, _, n in chunk])
-            self._stage(self.tokens, toks, torch.int32)
-            self._stage(self.slots, slots, torch.int32)
-            self.n_distinct = len({int(s) for s in slots if s >= 0})
+            row_slot, row_pos = kv.begin_rows([seq_ids[i] for i, _, _ in chunk], lens)
+            self.n_distinct = len({int(adapter_slots[i]) for i, _, _ in chunk if adapter_slots[i] >= 0})
             self.max_keys = max(p0 + n for _, _, n, p0 in passes)
-            self.row_slot[:T].copy_(row_slot)
-            self.row_pos[:T].copy_(row_pos)
             rows, dest, row_of = [], [], {}
             for (i, s, n), (_, r0, _, _) in zip(chunk, passes):
                 for k, w in enumerate(want[i]):
@@ -122,13 +139,19 @@ class EngineBase:
                             row_of[r] = len(rows)
                             rows.append(r)
                         dest.append((first_out[i] + k, row_of[r]))
+            self._stage_all((self.tokens, toks), (self.slots, np.repeat([adapter_slots[i] for i, _, _ in chunk], lens)),
+                            (self.row_slot, row_slot), (self.row_pos, row_pos), (self.last_rows, rows or [T - 1]))
             self._begin_prompt_pass(passes)
-            self._stage(self.last_rows, rows or [T - 1], torch.int32)
             lg, tk = self.forward(T, False, use_lora, self.last_rows, max(len(rows), 1))
             if rows:
-                to, src = torch.tensor(dest, device=dev).unbind(1)
-                out_logits[to] = lg[src]
-                out_tok[to] = tk[src]
+                d0, n = dest[0][0], len(rows)
+                if dest == [(d0 + k, k) for k in range(n)]:  # one row after the other, as in every plain prefill
+                    out_logits[d0:d0 + n].copy_(lg[:n])
+                    out_tok[d0:d0 + n].copy_(tk[:n])
+                else:
+                    to, src = torch.tensor(dest).pin_memory().to(dev, non_blocking=True).unbind(1)
+                    out_logits[to] = lg[src]
+                    out_tok[to] = tk[src]
             kv.end_forward()
             self._end_prompt_pass()
         self.check_status()  # (synchronises; prefill is not the latency-critical call)

@@ -56,7 +56,7 @@ class PagedCache:
         self._slot_of[sid] = slot
         self._n_pages_of[sid] = 0
         self._len_host[slot] = 0
-        self._push(self.seq_lens[slot:slot + 1], self._len_host[slot:slot + 1])
+        self.seq_lens[slot:slot + 1].zero_()  # (a fill: no staging buffer)
         return slot
 
     def _push(self, dst, src_np):
@@ -65,7 +65,7 @@ class PagedCache:
     def remove_sequence(self, sid):
         slot = self._slot_of.pop(sid)
         n = self._n_pages_of.pop(sid)
-        self._free.extend(int(p) for p in self._bt_host[slot, :n].tolist()[::-1])
+        self._free.extend(self._bt_host[slot, :n][::-1].tolist())
         self._free_slots.append(slot)
 
     def slot(self, sid):
@@ -80,37 +80,65 @@ class PagedCache:
 
     def reserve(self, sid, n_tokens):
         """Make sure pages exist for ``n_tokens`` total tokens of sequence ``sid``."""
+        self._push_pages(self._take_pages(sid, n_tokens))
+
+    def _take_pages(self, sid, n_tokens):
+        """The host side of :meth:`reserve`: what the device table lacks then, as a list of (slot, first entry, end)."""
         slot = self._slot_of[sid]
         need = (int(n_tokens) + self.page_size - 1) // self.page_size
         have = self._n_pages_of[sid]
         if need <= have:
-            return
+            return []
         if need > self.max_pages:
             raise RuntimeError(f"sequence {sid} needs {need} pages, block table holds {self.max_pages}")
         if need - have > len(self._free):
             raise RuntimeError("paged KV cache is out of pages")
-        for p in range(have, need):
-            self._bt_host[slot, p] = self._free.pop()
+        self._bt_host[slot, have:need] = self._free[:have - need - 1:-1]
+        del self._free[have - need:]
         self._n_pages_of[sid] = need
-        self._push(self.block_table[slot, have:need], self._bt_host[slot, have:need])
+        return [(slot, have, need)]
+
+    # one copy of the table's rows between the first and the last changed sequence (the host mirror is the table, so the
+    # others are written as they are) costs what a copy per sequence does up to about this many entries each
+    _ROWS_PER_COPY = 16384
+
+    def _push_pages(self, changed):
+        if not changed:
+            return
+        lo, hi = min(c[0] for c in changed), max(c[0] for c in changed) + 1
+        if len(changed) > 1 and (hi - lo) * self.max_pages <= self._ROWS_PER_COPY * len(changed):
+            self._push(self.block_table[lo:hi], self._bt_host[lo:hi])
+            return
+        for slot, have, need in changed:
+            self._push(self.block_table[slot, have:need], self._bt_host[slot, have:need])
 
     # -- the reference's forward protocol -------------------------------------------------------------
     def begin_forward(self, seq_ids, append_lens):
         """Reserve pages for the rows of this forward and return (row_slot, row_pos) device tensors:
         one row per appended token, sequences in the order given."""
+        rows = self.begin_rows(seq_ids, append_lens)
+        T = rows[0].size
+        both = np.zeros((2, (T + 63) // 64 * 64), dtype=np.int32)
+        both[:, :T] = rows
+        both = torch.from_numpy(both).pin_memory().to(self.device, non_blocking=True)
+        return both[0, :T], both[1, :T]
+
+    def begin_rows(self, seq_ids, append_lens):
+        """:meth:`begin_forward` for a caller that uploads the rows with others of its own: two int32 arrays on the host."""
         seq_ids = [int(s) for s in seq_ids]
         append_lens = [int(a) for a in append_lens]
-        slots, pos = [], []
-        for sid, a in zip(seq_ids, append_lens):
-            slot = self._slot_of[sid]
-            n0 = int(self._len_host[slot])
-            self.reserve(sid, n0 + a)
-            slots.extend([slot] * a)
-            pos.extend(range(n0, n0 + a))
+        slots = np.array([self._slot_of[s] for s in seq_ids], dtype=np.int32)
+        lens = np.array(append_lens, dtype=np.int64)
+        first = self._len_host[slots]
+        changed = []
+        try:
+            for sid, n in zip(seq_ids, (first + lens).tolist()):
+                changed += self._take_pages(sid, n)
+        finally:  # (sequences before one that finds no page keep what they got)
+            self._push_pages(changed)
         self._pending = (seq_ids, append_lens)
-        row_slot = torch.tensor(slots, dtype=torch.int32).pin_memory().to(self.device, non_blocking=True)
-        row_pos = torch.tensor(pos, dtype=torch.int32).pin_memory().to(self.device, non_blocking=True)
-        return row_slot, row_pos
+        start = first.astype(np.int64) - (np.cumsum(lens) - lens)  # position of a sequence's row r = start + r
+        return np.repeat(slots, lens), (np.arange(int(lens.sum())) + np.repeat(start, lens)).astype(np.int32)
 
     def end_forward(self):
         seq_ids, append_lens = self._pending

@@ -20,10 +20,16 @@ from __future__ import annotations
 
 from typing import Any
 
+import numpy as np
 import torch
 from torch import nn
 
 from . import ops
+
+
+def _address(linear):
+    w = linear._parameters.get("weight")
+    return (linear.weight if w is None else w).data_ptr()
 
 
 class MultiLoraLinear(nn.Module):
@@ -87,9 +93,11 @@ class MultiLoraLinear(nn.Module):
 
     # -- packing ------------------------------------------------------------------------------------------
     def _pack(self):
-        names = sorted(self.lora_A.keys())
-        key = tuple((n, self.lora_A[n].weight.data_ptr(), self.lora_B[n].weight.data_ptr(), self.scaling[n])
-                    for n in names) + (self.base_layer.weight.data_ptr(),)
+        """(key, stack, name -> slot, packed weight), rebuilt when a weight has moved.  Every forward compares the addresses of
+        all adapters: straight from the modules' own dicts, a module attribute costs ten times as much."""
+        A, B, scaling = self.lora_A._modules, self.lora_B._modules, self.scaling
+        names = sorted(A)
+        key = tuple([(n, _address(A[n]), _address(B[n]), scaling[n]) for n in names]) + (_address(self.base_layer),)
         if self._packed is not None and self._packed[0] == key:
             return self._packed
         dev = self.base_layer.weight.device
@@ -122,17 +130,16 @@ class MultiLoraLinear(nn.Module):
         cache = self._ctx.slot_cache if self._ctx is not None else None
         if cache is not None and key in cache:
             return cache[key]
-        t = torch.tensor(slots_per_batch_row, dtype=torch.int32).repeat_interleave(per_row).pin_memory() \
-            .to(device, non_blocking=True)
+        t = torch.from_numpy(np.repeat(np.array(slots_per_batch_row, dtype=np.int32), per_row)).pin_memory().to(device, non_blocking=True)
         if cache is not None:
             if len(cache) > 64:
                 cache.clear()
             cache[key] = t
         return t
 
-    def _run(self, x, slots_per_batch_row):
-        """x [B,S,in] (or [T,in]); one slot per leading row, shared by that row's S tokens."""
-        _, stack, _, Wp = self._pack()
+    def _run(self, x, slots_per_batch_row, packed=None):
+        """x [B,S,in] (or [T,in]); one slot per leading row, shared by that row's S tokens.  ``packed``: this call's _pack()."""
+        _, stack, _, Wp = packed or self._pack()
         lead = x.shape[:-1]
         x2 = x.reshape(-1, self.in_features)
         if x2.dtype != torch.bfloat16 or not x2.is_contiguous():
@@ -140,7 +147,7 @@ class MultiLoraLinear(nn.Module):
         slots = None
         if slots_per_batch_row is not None and stack is not None:
             slots = self._slot_tensor(slots_per_batch_row, x2.shape[0] // len(slots_per_batch_row), x2.device)
-        y = ops.linear(x2, Wp, stack if slots is not None else None, slots)
+        y = ops.linear(x2, Wp, stack if slots is not None else None, slots, with_shrink=True)
         if self.base_layer.bias is not None:
             y = y + self.base_layer.bias.to(y.dtype)
         y = y.reshape(*lead, self.out_features)
@@ -158,9 +165,10 @@ class MultiLoraLinear(nn.Module):
                 self.unmerge()
             return self._run(x, None)
         if adapter_names is not None:
-            _, _, slot_of, _ = self._pack()
+            packed = self._pack()
+            slot_of = packed[2]
             # "__base__" is peft's name for "no adapter on this row"
-            return self._run(x, [slot_of.get(n, -1) for n in adapter_names])
+            return self._run(x, [slot_of.get(n, -1) for n in adapter_names], packed)
         if self.merged:
             return self._run(x, None)
         active = [n for n in self.active_adapters if n in self.lora_A]
@@ -169,9 +177,9 @@ class MultiLoraLinear(nn.Module):
         if not active:
             return self._run(x, None)
         if len(active) == 1:
-            _, _, slot_of, _ = self._pack()
+            packed = self._pack()
             n_rows = x.shape[0] if x.dim() > 1 else 1
-            return self._run(x, [slot_of[active[0]]] * n_rows)
+            return self._run(x, [packed[2][active[0]]] * n_rows, packed)
         # several active adapters apply to every row: their deltas add, one pass per adapter
         _, stack, slot_of, Wp = self._pack()
         x2 = x.reshape(-1, self.in_features).to(torch.bfloat16).contiguous()

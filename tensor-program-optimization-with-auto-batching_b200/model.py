@@ -459,7 +459,7 @@ class Engine(EngineBase):
                  for sid, r0, n, p0 in chunk for off in range(0, n, 128)]
         self._n_pf_tiles = 0
         if self.tc_prefill and len(tiles) <= self.pf_tiles.shape[0]:
-            self._stage(self.pf_tiles.view(-1), np.asarray(tiles, dtype=np.int32).reshape(-1), torch.int32)
+            self._stage_all((self.pf_tiles.view(-1), tiles))
             self._n_pf_tiles = len(tiles)
 
     def _end_prompt_pass(self):

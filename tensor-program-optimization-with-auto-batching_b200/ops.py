@@ -16,12 +16,12 @@ from ._lib import check
 OUT_F32, SILU_MUL, FORCE_SIMT, W_PACKED, B_PACKED, SHARE_LORA_KERNEL, LORA_PER_ROW, B_SPLIT = 1, 2, 4, 8, 16, 32, 64, 128
 
 
-def _ptr(t):
-    return None if t is None else C.c_void_p(t.data_ptr())
+def _ptr(t):  # (plain numbers: the prototypes convert them)
+    return None if t is None else t.data_ptr()
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return torch.cuda.current_stream().cuda_stream
 
 
 def _need_cuda(*ts):

@@ -234,8 +234,7 @@ class RelidraEngine(PlainEngine):
     def _begin_prompt_pass(self, chunk):
         segs = [(self.kv.slot(sid), r0, n, p0) for sid, r0, n, p0 in chunk]
         tiles = [(s, r0 + off, min(128, n - off), p0 + off) for s, r0, n, p0 in segs for off in range(0, n, 128)]
-        for dst, v in ((self.segs, segs), (self.tiles, tiles)):
-            self._stage(dst.view(-1), np.asarray(v, dtype=np.int32).reshape(-1), torch.int32)
+        self._stage_all((self.segs.view(-1), segs), (self.tiles.view(-1), tiles))
         self._n_segs, self._n_tiles, self._max_seg = len(segs), len(tiles), max(n for _, _, n, _ in segs)
 
     def _end_prompt_pass(self):

@@ -17,7 +17,6 @@ from __future__ import annotations
 
 from dataclasses import dataclass
 
-import numpy as np
 import torch
 
 from . import ops
@@ -239,8 +238,7 @@ class TevudraEngine(PlainEngine):
             base += c
         if len(tiles) > self.tiles.shape[0] or len(segs) > self.segs.shape[0]:
             return
-        self._stage(self.tiles.view(-1), np.asarray(tiles, dtype=np.int32).reshape(-1), torch.int32)
-        self._stage(self.segs.view(-1), np.asarray(segs, dtype=np.int32).reshape(-1), torch.int32)
+        self._stage_all((self.tiles.view(-1), tiles), (self.segs.view(-1), segs))
         self._n_tiles, self._n_segs, self._ctx_rows, self._max_ctx = len(tiles), len(segs), base, max(ctx)
 
     def _end_prompt_pass(self):
