@@ -46,26 +46,7 @@ __global__ void __launch_bounds__(kExpThreads) lora_expand_rows_kernel(LinearArg
   const float* um = su + module_of(a, o) * a.r_max;
   const int n_chunks = (rank + 7) / 8;
   float acc = 0.f;
-  if (packed == 2) {
-    // split layout: slice j of this adapter is the [out, 8] block number ranks[n_adapters + slot] + j
-    const int first = a.ranks[a.n_adapters + slot];
-    const uint4* base = reinterpret_cast<const uint4*>(a.B_all) + (size_t)first * a.out + o;
-    for (int c0 = 0; c0 < n_chunks; c0 += 8) {  // up to 8 x 128-bit loads in flight
-      uint4 v[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c)
-        if (c0 + c < n_chunks) v[c] = ld_stream(base + (size_t)(c0 + c) * a.out);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        if (c0 + c < n_chunks) {
-          float bf[8];
-          unpack8(v[c], bf);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) acc = fmaf(um[(c0 + c) * 8 + e], bf[e], acc);
-        }
-      }
-    }
-  } else if (!packed) {
+  if (!packed) {
     const bf16* b = a.B_all + ((size_t)slot * a.out + o) * a.r_max;
     for (int c0 = 0; c0 < n_chunks; c0 += 8) {  // up to 8 x 128-bit loads in flight
       uint4 v[8];
@@ -119,6 +100,83 @@ __global__ void __launch_bounds__(kExpThreads) lora_expand_rows_kernel(LinearArg
     *y16 = __float2bfloat16_rn(y_new);
 }
 
+// The split layout by a CTA of its own per (row, 1024 output features).  What bounds it is HBM where every row brings its
+// adapter, if enough is in flight: the lookups slot -> rank and first slice -> B are paid once per 1024 features
+// instead of once per 256, and low ranks take several features per thread at a time, so that every thread keeps up to eight
+// 128-bit loads in flight whatever the rank.  Measured, projection with expand, ranks 8 / 16 / 32 / 64 in turn, against 256
+// features per CTA: 128 rows 5120 -> 15360 79 -> 69 us (38 of them the projection), 5120 -> 5120 40.1 -> 38.8, 64 rows
+// 4096 -> 12288 45 -> 41; one rank 16: 43 -> 37.
+constexpr int kExpSpan = 1024;
+
+template <int NC, int PER>  // 16-byte slices of a feature in flight, features of a thread at a time
+__device__ __forceinline__ void expand_span(const LinearArgs& a, const uint4* base, int n, const float* su, float scale, int t, int o0, int o1) {
+  const bool f32 = (a.flags & MLORA_OUT_F32) != 0;
+#pragma unroll 1
+  for (int ob = o0 + threadIdx.x; ob < o1; ob += kExpThreads * PER) {
+    float y[PER], acc[PER];
+    const float* um[PER];
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int o = min(ob + i * kExpThreads, o1 - 1);
+      const size_t at = (size_t)t * a.ldy + o;
+      y[i] = f32 ? reinterpret_cast<const float*>(a.y)[at] : __bfloat162float(reinterpret_cast<const bf16*>(a.y)[at]);
+      um[i] = su + module_of(a, o) * a.r_max;
+      acc[i] = 0.f;
+    }
+#pragma unroll 1
+    for (int c0 = 0; c0 < n; c0 += NC) {
+      uint4 v[PER][NC];
+#pragma unroll
+      for (int i = 0; i < PER; ++i) {
+        const int o = min(ob + i * kExpThreads, o1 - 1);
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          if (c0 + c < n) v[i][c] = ld_stream(base + (size_t)(c0 + c) * a.out + o);
+      }
+#pragma unroll
+      for (int i = 0; i < PER; ++i)
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+          if (c0 + c < n) {
+            float bf[8];
+            unpack8(v[i][c], bf);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[i] = fmaf(um[i][(c0 + c) * 8 + e], bf[e], acc[i]);
+          }
+    }
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int o = ob + i * kExpThreads;
+      if (o < o1) store_out(a, t, o, fmaf(acc[i], scale, y[i]));
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kExpThreads) lora_expand_split_kernel(LinearArgs a) {
+  __shared__ float su[kExpMaxRtot];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.y, slot = a.slots[t];
+  if (slot < 0 || slot >= a.n_adapters) return;  // (uniform)
+  const int first = a.ranks[a.n_adapters + slot];
+  const int rank = min(a.ranks[slot], a.r_max);
+  const float scale = a.scales[slot];
+  const int r_tot = a.r_max * a.n_mod;
+  for (int i = threadIdx.x; i < r_tot; i += kExpThreads) su[i] = a.u[(size_t)t * r_tot + i];
+  __syncthreads();
+  const int o0 = blockIdx.x * kExpSpan, o1 = min(a.out, o0 + kExpSpan);
+  const uint4* base = reinterpret_cast<const uint4*>(a.B_all) + (size_t)first * a.out;
+  const int n = (rank + 7) / 8;
+  if (n <= 1)
+    expand_span<1, 4>(a, base, n, su, scale, t, o0, o1);
+  else if (n <= 2)
+    expand_span<2, 4>(a, base, n, su, scale, t, o0, o1);
+  else if (n <= 4)
+    expand_span<4, 2>(a, base, n, su, scale, t, o0, o1);
+  else
+    expand_span<8, 1>(a, base, n, su, scale, t, o0, o1);
+}
+
 }  // namespace
 
 bool lora_expand_rows_supported(const LinearArgs& a) {
@@ -134,9 +192,15 @@ bool lora_expand_silu_supported(const LinearArgs& a) {
 }
 
 int launch_lora_expand_rows(const LinearArgs& a, cudaStream_t st) {
+  if (a.flags & MLORA_B_SPLIT) {
+    launch_pdl_if(pdl_enabled(), lora_expand_split_kernel, dim3((a.out + kExpSpan - 1) / kExpSpan, a.T), dim3(kExpThreads), 0, st, a);
+    count_launch();
+    MLORA_CHECK_LAUNCH("lora_expand_split_kernel");
+    return MLORA_OK;
+  }
   dim3 grid((a.out + kExpThreads - 1) / kExpThreads, a.T);
   launch_pdl_if(pdl_enabled(), lora_expand_rows_kernel, grid, dim3(kExpThreads), 0, st, a,
-                (a.flags & MLORA_B_SPLIT) ? 2 : (a.flags & MLORA_B_PACKED) ? 1 : 0);
+                (a.flags & MLORA_B_PACKED) ? 1 : 0);
   count_launch();
   MLORA_CHECK_LAUNCH("lora_expand_rows_kernel");
   return MLORA_OK;
