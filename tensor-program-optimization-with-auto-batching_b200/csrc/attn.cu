@@ -426,6 +426,74 @@ __global__ void __launch_bounds__(256) kv_append_rope_kernel(bf16* __restrict__ 
   }
 }
 
+// The same values in 16-byte pieces, where the key pages are aligned to that: a thread takes 8 dimensions of the first half of a
+// head and the 8 that rotate with them, and requests its pieces of two heads and of two value heads before it waits for the
+// row's sines and cosines (computed once per row, not once per thread) and its page.  Bound by HBM: a row is read and
+// written once.  Measured, 8192 rows, 32 + 2 x 32 heads of 128: 108 -> 80 us (403 MB, 5.0 TB/s); 1000 rows of 40 heads 17.9 -> 14.6.
+constexpr int kRope16Threads = 256;
+constexpr int kRope16MaxD = 128;
+
+__global__ void __launch_bounds__(kRope16Threads) kv_append_rope16_kernel(bf16* __restrict__ qkv, int64_t ld, bf16* __restrict__ k_pages,
+                                                                          bf16* __restrict__ v_pages,
+                                                                          const int32_t* __restrict__ block_table, int max_pages,
+                                                                          const int32_t* __restrict__ row_slot,
+                                                                          const int32_t* __restrict__ row_pos, int Hq, int Hkv, int D,
+                                                                          int PS, float theta) {
+  __shared__ float s_sn[kRope16MaxD / 2], s_cs[kRope16MaxD / 2];
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x, tid = threadIdx.x;
+  const int slot = row_slot[t], pos = row_pos[t];
+  if (pos < 0 || pos / PS >= max_pages) return;  // no block-table entry for this position: nothing is written
+  bf16* row = qkv + (size_t)t * ld;
+  const bf16* vsrc = row + (size_t)(Hq + Hkv) * D;
+  const int half = D / 2, per_head = half / 8, n_rot = (Hq + Hkv) * per_head, per_v = D / 8, n_v = Hkv * per_v;
+  uint4 lo[2], hi[2], val[2];
+  auto load = [&](int base) {
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int u = base + b * kRope16Threads;
+      if (u < n_rot) {
+        const bf16* p = row + (size_t)(u / per_head) * D + (u % per_head) * 8;
+        lo[b] = *reinterpret_cast<const uint4*>(p);
+        hi[b] = *reinterpret_cast<const uint4*>(p + half);
+      }
+      if (u < n_v) val[b] = *reinterpret_cast<const uint4*>(vsrc + (size_t)u * 8);
+    }
+  };
+  load(tid);
+  const int page = block_table[(size_t)slot * max_pages + pos / PS];
+  for (int i = tid; i < half; i += kRope16Threads) sincosf((float)pos * rope_inv_freq(theta, i, D), &s_sn[i], &s_cs[i]);
+  __syncthreads();
+  for (int base = tid; base < max(n_rot, n_v);) {
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const int u = base + b * kRope16Threads;
+      if (u < n_rot) {
+        const int head = u / per_head, i = (u % per_head) * 8;
+        float x1[8], x2[8], r1[8], r2[8];
+        unpack8(lo[b], x1);
+        unpack8(hi[b], x2);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const float sn = s_sn[i + e], cs = s_cs[i + e];
+          r1[e] = x1[e] * cs - x2[e] * sn;
+          r2[e] = x2[e] * cs + x1[e] * sn;
+        }
+        bf16* dst = (head < Hq ? row + (size_t)head * D : k_pages + (((size_t)page * Hkv + (head - Hq)) * PS + pos % PS) * D) + i;
+        *reinterpret_cast<uint4*>(dst) = pack8(r1);
+        *reinterpret_cast<uint4*>(dst + half) = pack8(r2);
+      }
+      if (u < n_v) {
+        const int head = u / per_v;
+        *reinterpret_cast<uint4*>(v_pages + (((size_t)page * Hkv + head) * PS + pos % PS) * D + (u % per_v) * 8) = val[b];
+      }
+    }
+    base += 2 * kRope16Threads;
+    if (base < max(n_rot, n_v)) load(base);
+  }
+}
+
 int pick_splits(int T, int Hq, int max_pages) {
   const int base = T * Hq;
   if (base >= 592) return 1;  // >= 4 CTAs on each of the 148 SMs already
@@ -463,9 +531,9 @@ extern "C" int mlora_kv_append_rope(void* d_qkv, int64_t ld, void* d_k_pages, vo
                 "kv_append_rope: null pointer");
   MLORA_REQUIRE(ld % 8 == 0 && aligned16(d_qkv) && aligned16(d_v_pages), "kv_append_rope: alignment");
   if (T == 0) return MLORA_OK;
-  launch_pdl(kv_append_rope_kernel, T, 256, 0, (cudaStream_t)stream, (bf16*)d_qkv, ld, (bf16*)d_k_pages, (bf16*)d_v_pages,
-                                                             d_block_table, max_pages, d_row_slot, d_row_pos, Hq, Hkv,
-                                                             D, page_size, rope_theta);
+  const bool wide = aligned16(d_k_pages);  // (qkv and the value pages are: checked above)
+  launch_pdl(wide ? kv_append_rope16_kernel : kv_append_rope_kernel, T, kRope16Threads, 0, (cudaStream_t)stream, (bf16*)d_qkv, ld,
+             (bf16*)d_k_pages, (bf16*)d_v_pages, d_block_table, max_pages, d_row_slot, d_row_pos, Hq, Hkv, D, page_size, rope_theta);
   count_launch();
   MLORA_CHECK_LAUNCH("kv_append_rope_kernel");
   return MLORA_OK;
