@@ -18,7 +18,8 @@
 // columns each) and fill each other's gaps; a CTA's own copies are off the chain: K of the next block is fetched from the
 // moment S = Q K^T has read it, V from the moment P V has.  CTAs of late tiles (most keys) start first.
 // Measured (32 heads of 128, keys and values dense, CUDA events), one buffer of K / V and O in registers -> this:
-// 2 x 4096 rows 590 -> 354 us (777 TFLOP/s), 16 x 512 148 -> 104, 64 x 128 97 -> 74, 1 x 8192 1085 -> 639 (860).
+// 2 x 4096 rows 590 -> 354 us (777 TFLOP/s), 16 x 512 148 -> 104, 64 x 128 97 -> 74, 1 x 8192 1085 -> 639 (860); from pages
+// 358 us where they lie in order (eight per copy), 435 shuffled.
 // Every wait is bounded; a CTA that gives up writes zeros.
 #include <math.h>
 
@@ -59,6 +60,7 @@ struct PfArgs {
   int chunk;        // > 0: a row sees only positions of its own chunk of this many (counted from position 0)
   const float* sink;  // [Hq] or NULL: a logit per head that only enters the softmax's sum
   int n_tiles;
+  int runs;         // paged form: the maps of eight pages are there (pages of 16)
 };
 
 // NK, NV: query/key and value size of a head in 64s.  PAGED: keys and values come 16 at a time through the block table,
@@ -68,6 +70,8 @@ template <int NK, int NV, bool PAGED>
 __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q,
                                                                          const __grid_constant__ CUtensorMap map_k,
                                                                          const __grid_constant__ CUtensorMap map_v,
+                                                                         const __grid_constant__ CUtensorMap map_k8,
+                                                                         const __grid_constant__ CUtensorMap map_v8,
                                                                          PfArgs a) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* sq = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -105,6 +109,10 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
     tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_k);
     tma_prefetch_desc(&map_v);
+    if (PAGED && a.runs) {
+      tma_prefetch_desc(&map_k8);
+      tma_prefetch_desc(&map_v8);
+    }
   }
   if (warp == 4) tmem_alloc(&tmem_slot, 256);
   tc_fence_before();
@@ -131,8 +139,22 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
       return PAGED && lane < kTile / kPS && pg < n_pages
                  ? ((bt[pg / a.page_parts] * a.Hkv + kvh) * a.page_parts + pg % a.page_parts) * kPS : -kPS;
     };
-    auto copy = [&](int kb, int page, uint8_t* dst, const CUtensorMap* map, uint64_t* bar, int parts, int col, uint32_t more) {
+    auto copy = [&](int kb, int page, uint8_t* dst, const CUtensorMap* map, const CUtensorMap* map8, uint64_t* bar, int parts, int col,
+                    uint32_t more) {
       const int valid = PAGED ? min(kTile / kPS, n_pages - key0 / kPS - kb * (kTile / kPS)) : 0;
+      if (PAGED && a.runs && valid == kTile / kPS) {
+        // eight pages one after the other in the pool, as a pool that has not been churned hands them out: one copy per
+        // 64-column part instead of eight (copies of 2 KB are bound by their number)
+        const int first = __shfl_sync(0xffffffffu, page, 0);
+        if (__all_sync(0xffffffffu, lane >= kTile / kPS || page == first + lane * a.Hkv * kPS)) {
+          if (lane == 0) {
+            mbar_expect_tx(bar, (uint32_t)(parts * kSub) + more);
+            for (int j = 0; j < parts; ++j) tma_load_4d(dst + j * kSub, map8, j * 64, 0, kvh, (first / kPS - kvh) / a.Hkv, bar);
+          }
+          __syncwarp();
+          return;
+        }
+      }
       if (lane == 0) {
         mbar_expect_tx(bar, (PAGED ? (uint32_t)(valid * parts * kPS * 128) : (uint32_t)(parts * kSub)) + more);
         if constexpr (!PAGED)  // rows past the sequence's last key belong to the next one (or are zeros): masked
@@ -145,10 +167,10 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
     };
     const int k_col = h * NK * 64, v_col = a.v_col + h * NV * 64;
     int page = page_of(0), page_next = page_of(1);
-    copy(0, page, sk, &map_k, &kbar, NK, k_col, NK * kSub);
+    copy(0, page, sk, &map_k, &map_k8, &kbar, NK, k_col, NK * kSub);
     if (lane == 0)
       for (int j = 0; j < NK; ++j) tma_load_2d(sq + j * kSub, &map_q, k_col + j * 64, row0, &kbar);
-    copy(0, page, sv, &map_v, &vbar, NV, v_col, 0);
+    copy(0, page, sv, &map_v, &map_v8, &vbar, NV, v_col, 0);
     for (int kb = 0; kb < n_blocks; ++kb) {
       const uint32_t par = kb & 1;
       if (!wait(&kbar, par)) break;
@@ -165,13 +187,13 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
       }
       if (kb > 0) {  // V's place is free once the P V before has retired (as it has when this S retires)
         if (!wait(&obar, par ^ 1)) break;
-        copy(kb, page, sv, &map_v, &vbar, NV, v_col, 0);
+        copy(kb, page, sv, &map_v, &map_v8, &vbar, NV, v_col, 0);
       }
       if (kb + 1 < n_blocks) {
         if (!wait(&sbar, par)) break;
         page = page_next;
         page_next = page_of(kb + 2);
-        copy(kb + 1, page, sk, &map_k, &kbar, NK, k_col, 0);
+        copy(kb + 1, page, sk, &map_k, &map_k8, &kbar, NK, k_col, 0);
       }
       if (!wait(&vbar, par) || !wait(&pbar, par)) break;
       if (lane == 0) {
@@ -304,8 +326,23 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
   if (warp == 4) tmem_dealloc(tmem_base, 256);
 }
 
+// Pages [n_pages][Hkv][16][D] with a box of eight pages of one head, 64 columns: the same 128 rows of 128 bytes in shared memory
+// that eight copies of a page write.
+int make_pages_map(CUtensorMap* m, const void* ptr, int n_pages, int Hkv, int D) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(MLORA_ECUDA, "prefill_attention: cuTensorMapEncodeTiled is not available from this driver");
+  cuuint64_t dims[4] = {(cuuint64_t)D, (cuuint64_t)kPS, (cuuint64_t)Hkv, (cuuint64_t)n_pages};
+  cuuint64_t strides[3] = {(cuuint64_t)D * 2, (cuuint64_t)kPS * D * 2, (cuuint64_t)Hkv * kPS * D * 2};
+  cuuint32_t box[4] = {64, (cuuint32_t)kPS, 1, (cuuint32_t)(kTile / kPS)};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(MLORA_ECUDA, "prefill_attention: cuTensorMapEncodeTiled (pages) failed with %d", (int)r);
+  return MLORA_OK;
+}
+
 template <int NK, int NV, bool PAGED>
-int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, PfArgs a, int n_tiles, cudaStream_t st) {
+int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mk8, const CUtensorMap& mv8, PfArgs a, int n_tiles, cudaStream_t st) {
   if ((long long)n_tiles * a.Hq > 2147483647ll) return fail(MLORA_ESIZE, "prefill_attention: too many tiles x heads");
   a.n_tiles = n_tiles;
   constexpr int smem = (2 * NK + NV) * kSub + 1024;  // Q, K, V
@@ -317,7 +354,7 @@ int launch_prefill(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorM
     if (e != cudaSuccess) return fail(MLORA_ECUDA, "prefill_attention: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     attr_done.fetch_or(1ull << (dev & 63), std::memory_order_release);
   }
-  prefill_attn_tc_kernel<NK, NV, PAGED><<<(unsigned)((long long)n_tiles * a.Hq), kPfThreads, smem, st>>>(mq, mk, mv, a);
+  prefill_attn_tc_kernel<NK, NV, PAGED><<<(unsigned)((long long)n_tiles * a.Hq), kPfThreads, smem, st>>>(mq, mk, mv, mk8, mv8, a);
   count_launch();
   MLORA_CHECK_LAUNCH("prefill_attn_tc_kernel");
   return MLORA_OK;
@@ -352,9 +389,17 @@ extern "C" int mlora_prefill_attention_masked(const void* d_q, int64_t ld, const
   rc = make_map(&mv, d_v_pages, (long long)n_pages_total * Hkv * page_size, D, D, kPS, 64);
   if (rc) return rc;
   PfArgs a{d_block_table, max_pages, d_tiles, Hq, Hkv, (bf16*)d_out, ld_out, d_status, scale, nullptr, 0, 0,
-           page_size / kPS, chunk, d_sink};
-  return D == 64 ? launch_prefill<1, 1, true>(mq, mk, mv, a, n_tiles, (cudaStream_t)stream)
-                 : launch_prefill<2, 2, true>(mq, mk, mv, a, n_tiles, (cudaStream_t)stream);
+           page_size / kPS, chunk, d_sink, 0, 0};
+  CUtensorMap mk8 = mk, mv8 = mv;
+  if (page_size == kPS) {
+    rc = make_pages_map(&mk8, d_k_pages, n_pages_total, Hkv, D);
+    if (rc) return rc;
+    rc = make_pages_map(&mv8, d_v_pages, n_pages_total, Hkv, D);
+    if (rc) return rc;
+    a.runs = 1;
+  }
+  return D == 64 ? launch_prefill<1, 1, true>(mq, mk, mv, mk8, mv8, a, n_tiles, (cudaStream_t)stream)
+                 : launch_prefill<2, 2, true>(mq, mk, mv, mk8, mv8, a, n_tiles, (cudaStream_t)stream);
 }
 
 extern "C" int mlora_prefill_attention(const void* d_qkv, int64_t ld, const void* d_k_pages, const void* d_v_pages,
@@ -386,10 +431,10 @@ extern "C" int mlora_prefill_attention_dense(const void* d_q, int64_t ld, const 
   if (rc) return rc;
   rc = make_map(&mkv, d_kv, kv_rows, v_col + H * Dv, ld_kv, kTile, 64);
   if (rc) return rc;
-  PfArgs a{nullptr, 0, d_tiles, H, H, (bf16*)d_out, ld_out, d_status, scale, (const bf16*)d_gate, ld_gate, v_col, 1, 0, nullptr};
+  PfArgs a{nullptr, 0, d_tiles, H, H, (bf16*)d_out, ld_out, d_status, scale, (const bf16*)d_gate, ld_gate, v_col, 1, 0, nullptr, 0, 0};
   cudaStream_t st = (cudaStream_t)stream;
-  if (Dk == 64 && Dv == 64) return launch_prefill<1, 1, false>(mq, mkv, mkv, a, n_tiles, st);
-  if (Dk == 64) return launch_prefill<1, 2, false>(mq, mkv, mkv, a, n_tiles, st);
-  if (Dv == 64) return launch_prefill<2, 1, false>(mq, mkv, mkv, a, n_tiles, st);
-  return launch_prefill<2, 2, false>(mq, mkv, mkv, a, n_tiles, st);
+  if (Dk == 64 && Dv == 64) return launch_prefill<1, 1, false>(mq, mkv, mkv, mkv, mkv, a, n_tiles, st);
+  if (Dk == 64) return launch_prefill<1, 2, false>(mq, mkv, mkv, mkv, mkv, a, n_tiles, st);
+  if (Dv == 64) return launch_prefill<2, 1, false>(mq, mkv, mkv, mkv, mkv, a, n_tiles, st);
+  return launch_prefill<2, 2, false>(mq, mkv, mkv, mkv, mkv, a, n_tiles, st);
 }

@@ -44,3 +44,36 @@ def test_scores_that_grow(growth, lens, Dk, Dv):
         got = out[base:base + n].double()
         assert ((got - want).abs() / want).max().item() < 2.0 ** -7
         base += n
+
+
+# pages of a sequence one after the other in the pool are fetched eight at a time: the same bytes as page by page
+@pytest.mark.parametrize("n", [1, 112, 128, 129, 640, 1000])
+@pytest.mark.parametrize("D,Hq,Hkv", [(128, 4, 2), (64, 3, 3)])
+def test_pages_in_runs_and_scattered(n, D, Hq, Hkv):
+    ops = load("ops")
+    g = torch.Generator(device="cuda").manual_seed(n)
+    pages = -(-n // 16)
+    q = torch.randn(n, Hq * D, generator=g, device="cuda").bfloat16()
+    k, v = (torch.full((3 * pages, Hkv, 16, D), float("nan"), device="cuda").bfloat16() for _ in range(2))
+    rows = torch.randn(2, n, Hkv, D, generator=g, device="cuda").bfloat16()
+    tables = [torch.arange(pages) + pages, torch.randperm(3 * pages, generator=torch.Generator().manual_seed(n))[:pages],
+              torch.arange(pages).flip(0), torch.arange(pages) * 2]
+    tables.append(tables[0].clone())
+    tables[4][pages // 2:] += 1  # a run that breaks off inside a block
+    tiles = torch.tensor([(0, o, min(128, n - o), o) for o in range(0, n, 128)], dtype=torch.int32, device="cuda")
+    outs = []
+    for table in tables:
+        k.fill_(float("nan")), v.fill_(float("nan"))
+        at = table.cuda()[torch.arange(n, device="cuda") // 16], torch.arange(n, device="cuda") % 16
+        k[at[0], :, at[1]], v[at[0], :, at[1]] = rows[0], rows[1]
+        out = torch.zeros(n, Hq * D, device="cuda").bfloat16()
+        status = torch.zeros(1, dtype=torch.int32, device="cuda")
+        ops.prefill_attention_masked(q, k, v, table[None].to(torch.int32).cuda(), tiles, len(tiles), Hq, D ** -0.5, out, status=status)
+        assert int(status) == 0
+        outs.append(out)
+    s = torch.einsum("qhd,khd->hqk", q.view(n, Hq, D).double(), rows[0].double().repeat_interleave(Hq // Hkv, 1)) * D ** -0.5
+    s = s.masked_fill(torch.ones(n, n, dtype=torch.bool, device="cuda").triu(1), float("-inf"))
+    want = torch.einsum("hqk,khd->qhd", torch.softmax(s, -1), rows[1].double().repeat_interleave(Hq // Hkv, 1)).flatten(1)
+    assert ((outs[0].double() - want).norm() / want.norm()).item() < 2.0 ** -7  # two roundings to bf16, as above
+    for o in outs[1:]:
+        assert torch.equal(o, outs[0])
