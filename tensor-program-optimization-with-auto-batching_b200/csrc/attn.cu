@@ -362,6 +362,7 @@ __global__ void __launch_bounds__(128) paged_attn_kernel(AttnArgs a) {
 }
 
 // grid (Hq, T), D threads: combine the n_splits partial results of one (row, head).
+constexpr int kMergeAtOnce = 16;
 __global__ void attn_merge_kernel(const float* __restrict__ work, int Hq, int D, int n_splits,
                                   bf16* __restrict__ out, int64_t ld_out) {
   pdl_launch_dependents();
@@ -369,6 +370,32 @@ __global__ void attn_merge_kernel(const float* __restrict__ work, int Hq, int D,
   const int h = blockIdx.x, t = blockIdx.y, d = threadIdx.x;
   const float* w = work + ((size_t)t * Hq + h) * n_splits * (D + 2);
   float M = -INFINITY;
+  if (n_splits <= kMergeAtOnce) {
+    // the splits that the automatic choice makes: everything in one round trip (it is nothing else; 5.0 -> 2.9 us at 16 splits), summed in the same order
+    float ms[kMergeAtOnce], ls[kMergeAtOnce], os[kMergeAtOnce];
+#pragma unroll
+    for (int s = 0; s < kMergeAtOnce; ++s) {
+      const bool in = s < n_splits;
+      const float* ws = w + (size_t)(in ? s : 0) * (D + 2);
+      ms[s] = in ? ws[D] : -INFINITY;
+      ls[s] = in ? ws[D + 1] : 0.f;
+      os[s] = in ? ws[d] : 0.f;
+    }
+#pragma unroll
+    for (int s = 0; s < kMergeAtOnce; ++s) M = fmaxf(M, ms[s]);
+    float L = 0.f, O = 0.f;
+    if (M != -INFINITY) {
+#pragma unroll
+      for (int s = 0; s < kMergeAtOnce; ++s) {
+        if (s >= n_splits) break;
+        const float c = (ms[s] == -INFINITY) ? 0.f : exp2f(ms[s] - M);
+        L = fmaf(ls[s], c, L);
+        O = fmaf(os[s], c, O);
+      }
+    }
+    out[(size_t)t * ld_out + h * D + d] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
+    return;
+  }
   for (int s = 0; s < n_splits; ++s) M = fmaxf(M, w[(size_t)s * (D + 2) + D]);
   float L = 0.f, O = 0.f;
   if (M != -INFINITY) {
