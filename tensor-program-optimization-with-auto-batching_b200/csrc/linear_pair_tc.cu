@@ -51,15 +51,6 @@ struct PairParams {
 };
 
 // ---- pair-wide PTX -----------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // the even CTA's copy of a shared-memory object, as a shared::cluster address
 __device__ __forceinline__ uint32_t lead_addr(const void* p) {
   uint32_t r;

@@ -9,10 +9,17 @@
 // in the output write.  When the distinct adapters of a tile need more than the accumulator / stage
 // budget they are processed in passes, each re-streaming the token tile (it is L2 resident).
 //
+// Few tiles (prompts of a few hundred to a few thousand rows) leave most of the chip idle, and one CTA's chain of k-blocks is
+// the time: the CTAs of a cluster take a share of the k-blocks each (`splits`), leave their partial rows in shared memory --
+// the ring, which is free by then -- and add them up in rank order through distributed shared memory, each CTA its part of
+// the rows.  A tile with more adapters than one pass holds is left to the first CTA.  Measured, one CTA per tile -> shared (us): 1000 rows of 4096, rank 16 on q/k/v 39.6 -> 14.8 (8 CTAs a tile),
+// 4096 rows 32.8 -> 16.9 (4), 8192 rows 33.5 -> 23.3 (2), 8192 rows of 11008, rank 64 76.5 -> 48.0; 16384 rows, not shared, 35.6.
+//
 // 192 threads: warp 0 = TMA producer (one thread), warp 1 = MMA issuer (one thread), warps 2..5 =
 // output (one TMEM lane = one token row per thread).  Every wait is bounded; when one expires the CTA
 // stops, writes NaN to its rows of u (so the failure cannot go unnoticed downstream) and leaves after
 // its copies in flight have landed and its TMEM is freed.
+#include <math.h>
 #include <stdlib.h>
 
 #include <atomic>
@@ -34,6 +41,7 @@ struct ShrinkParams {
   int T, r_tot, n_pad, n_adapters, k_blocks;
   int segs_per_pass;  // adapters whose accumulators / operand tiles fit at once
   int ring_bytes, tmem_cols;
+  int splits;  // CTAs of a cluster that share a tile (grid y)
 };
 
 __global__ void __launch_bounds__(kShrinkThreads, 1) lora_shrink_tc_kernel(const __grid_constant__ CUtensorMap map_x,
@@ -102,7 +110,12 @@ __global__ void __launch_bounds__(kShrinkThreads, 1) lora_shrink_tc_kernel(const
   }
   __syncthreads();
   const uint32_t tmem_base = tmem_slot;
-  const int n_pass = (n_seg + p.segs_per_pass - 1) / p.segs_per_pass;
+  float4* part = reinterpret_cast<float4*>(ring);  // [r_tot / 4][128 rows]
+  const int all_passes = (n_seg + p.segs_per_pass - 1) / p.segs_per_pass;
+  const int rank = p.splits > 1 ? (int)cluster_rank() : 0;
+  const bool split = p.splits > 1 && all_passes == 1;          // (the same in every CTA of the cluster)
+  const int n_pass = split || rank == 0 ? all_passes : 0;
+  const int kb0 = split ? rank * p.k_blocks / p.splits : 0, kb1 = split ? (rank + 1) * p.k_blocks / p.splits : p.k_blocks;
   const int a_tile = p.n_pad * 128;  // bytes of one adapter's operand tile in a stage
   // A stage holds the token tile and the operand tiles of the adapters THIS tile has (usually one: prompt rows of a
   // request are contiguous), so the ring is as deep as the shared memory allows: the kernel is a chain of L2 round trips
@@ -117,7 +130,7 @@ __global__ void __launch_bounds__(kShrinkThreads, 1) lora_shrink_tc_kernel(const
     bool ok = true;
     for (int ps = 0; ps < n_pass && ok; ++ps) {
       const int j0 = ps * p.segs_per_pass, nj = min(p.segs_per_pass, n_seg - j0);
-      for (int kb = 0; kb < p.k_blocks; ++kb, ++g) {
+      for (int kb = kb0; kb < kb1; ++kb, ++g) {
         const int s = g % stages, round = g / stages;
         if (!mbar_wait(&empty_bar[s], (round & 1) ^ 1, &s_abort)) {
           s_abort = 1;
@@ -153,7 +166,7 @@ __global__ void __launch_bounds__(kShrinkThreads, 1) lora_shrink_tc_kernel(const
         }
         tc_fence_after();
       }
-      for (int kb = 0; kb < p.k_blocks; ++kb, ++g) {
+      for (int kb = kb0; kb < kb1; ++kb, ++g) {
         const int s = g % stages, round = g / stages;
         if (!mbar_wait(&full_bar[s], round & 1, &s_abort)) {
           s_abort = 1;
@@ -167,7 +180,7 @@ __global__ void __launch_bounds__(kShrinkThreads, 1) lora_shrink_tc_kernel(const
           const uint64_t bdesc = make_smem_desc(st + kXTile + j * a_tile);
           const uint32_t d = tmem_base + (uint32_t)(j * p.n_pad);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) umma_bf16(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+          for (int k = 0; k < BK / 16; ++k) umma_bf16(d, adesc + 2 * k, bdesc + 2 * k, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
         }
         umma_commit(&empty_bar[s]);
       }
@@ -178,7 +191,7 @@ __global__ void __launch_bounds__(kShrinkThreads, 1) lora_shrink_tc_kernel(const
     const int row = (warp & 3) * 32 + lane, t = t0 + row;
     const int my = s_seg[row];
     float* ur = p.u + (size_t)t * p.r_tot;
-    if (t < p.T && my < 0)
+    if (!split && rank == 0 && t < p.T && my < 0)
       for (int c = 0; c < p.r_tot; c += 4) *reinterpret_cast<float4*>(ur + c) = make_float4(0.f, 0.f, 0.f, 0.f);
     bool ok = true;
     for (int ps = 0; ps < n_pass && ok; ++ps) {
@@ -199,7 +212,13 @@ __global__ void __launch_bounds__(kShrinkThreads, 1) lora_shrink_tc_kernel(const
         for (int c0 = 0; c0 < p.r_tot; c0 += 16) {
           float v[32];
           tmem_ld16(taddr + c0, v);
-          if (mine && t < p.T) {
+          if (split) {  // every MMA and copy of this CTA has retired: the ring is free
+            if (mine) {
+#pragma unroll
+              for (int c = 0; c < 16; c += 4)
+                if (c0 + c < p.r_tot) part[(c0 + c) / 4 * kTok + row] = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+            }
+          } else if (mine && t < p.T) {
 #pragma unroll
             for (int c = 0; c < 16; c += 4)
               if (c0 + c < p.r_tot) *reinterpret_cast<float4*>(ur + c0 + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
@@ -212,7 +231,27 @@ __global__ void __launch_bounds__(kShrinkThreads, 1) lora_shrink_tc_kernel(const
     }
   }
   __syncthreads();
-  if (s_abort && warp >= 2) {
+  if (p.splits > 1) {
+    if (split && s_abort && warp >= 2)  // (a NaN in a share makes the row's sums NaN)
+      for (int c = 0; c < p.r_tot / 4; ++c) part[c * kTok + (warp & 3) * 32 + lane] = make_float4(NAN, NAN, NAN, NAN);
+    cluster_sync();
+    if (split) {
+      const int rows = kTok / p.splits, r0 = rank * rows;
+      for (int i = tid; i < rows * (p.r_tot / 4); i += kShrinkThreads) {
+        const int row = r0 + i % rows, c = i / rows, t = t0 + row;
+        if (t >= p.T) continue;
+        float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s_seg[row] >= 0)
+          for (int q = 0; q < p.splits; ++q) {
+            const float4 v = ld_cluster4(&part[c * kTok + row], q);
+            sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
+          }
+        *reinterpret_cast<float4*>(p.u + (size_t)t * p.r_tot + c * 4) = sum;
+      }
+    }
+    cluster_sync();  // nobody leaves while its share is being read
+  }
+  if (!split && rank == 0 && s_abort && warp >= 2) {
     const int t = t0 + (warp & 3) * 32 + lane;
     if (t < p.T)
       for (int c = 0; c < p.r_tot; ++c) p.u[(size_t)t * p.r_tot + c] = __int_as_float(0x7fc00000);
@@ -264,7 +303,25 @@ int launch_lora_shrink_tc(const void* x, int64_t ldx, const void* A_all, const i
     if (e != cudaSuccess) return fail(MLORA_ECUDA, "lora_shrink: cudaFuncSetAttribute: %s", cudaGetErrorString(e));
     attr_done.fetch_or(1ull << (dev & 63), std::memory_order_release);
   }
-  launch_pdl_if(pdl_enabled_shrink(), lora_shrink_tc_kernel, dim3((T + kTok - 1) / kTok), dim3(kShrinkThreads), smem, st, mx, ma, p);
+  // as many CTAs per tile as the chip holds, down to eight k-blocks each
+  const int tiles = (T + kTok - 1) / kTok;
+  p.splits = 1;
+  while (p.splits < 8 && tiles * p.splits * 2 <= 148 && p.k_blocks >= p.splits * 16) p.splits *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles, p.splits);
+  cfg.blockDim = dim3(kShrinkThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = p.splits;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled_shrink() ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, lora_shrink_tc_kernel, mx, ma, p);
   count_launch();
   MLORA_CHECK_LAUNCH("lora_shrink_tc_kernel");
   return MLORA_OK;
