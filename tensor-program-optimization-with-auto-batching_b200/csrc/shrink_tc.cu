@@ -1,7 +1,7 @@
 // LoRA shrink at prefill sizes as a segmented grouped GEMM on the 5th-generation tensor cores
 // (tcgen05 + TMEM), fed by TMA:   u[t, :] = A_all[slot[t]] (r_tot x in) . x[t, :]
 //
-// One CTA per tile of 128 token rows.  The token tile is the M operand (128 TMEM lanes = 128 tokens);
+// One CTA (or a cluster of them, below) per tile of 128 token rows.  The token tile is the M operand (128 TMEM lanes = 128 tokens);
 // for every DISTINCT adapter among the tile's rows the adapter's A matrix (r_tot rows, padded to a
 // multiple of 16) is an N operand with its own accumulator columns, so a tile whose rows all use one
 // adapter (the usual case: prompt rows are contiguous per request) costs one pass over x, and a mixed
@@ -12,8 +12,9 @@
 // Few tiles (prompts of a few hundred to a few thousand rows) leave most of the chip idle, and one CTA's chain of k-blocks is
 // the time: the CTAs of a cluster take a share of the k-blocks each (`splits`), leave their partial rows in shared memory --
 // the ring, which is free by then -- and add them up in rank order through distributed shared memory, each CTA its part of
-// the rows.  A tile with more adapters than one pass holds is left to the first CTA.  Measured, one CTA per tile -> shared (us): 1000 rows of 4096, rank 16 on q/k/v 39.6 -> 14.8 (8 CTAs a tile),
-// 4096 rows 32.8 -> 16.9 (4), 8192 rows 33.5 -> 23.3 (2), 8192 rows of 11008, rank 64 76.5 -> 48.0; 16384 rows, not shared, 35.6.
+// the rows.  A tile with more adapters than one pass holds is left to the first CTA.  Measured, one CTA per tile -> shared (us):
+// 1000 rows of 4096, rank 16 on q/k/v 39.6 -> 14.8 (8 CTAs a tile), 4096 rows 32.8 -> 16.9 (4), 8192 rows 33.5 -> 23.3 (2),
+// 8192 rows of 11008, rank 64 76.5 -> 48.0; 16384 rows, not shared, 35.6.
 //
 // 192 threads: warp 0 = TMA producer (one thread), warp 1 = MMA issuer (one thread), warps 2..5 =
 // output (one TMEM lane = one token row per thread).  Every wait is bounded; when one expires the CTA
