@@ -5,25 +5,29 @@
 // One CTA = one tile of up to 128 consecutive prompt rows of ONE sequence x one head.  Per block of 128 keys:
 //   S = Q K^T      tcgen05.mma, M = 128 queries, N = 128 keys, K = head_dim 128; Q and K both K-major in 128-byte-swizzled
 //                  shared memory -- Q by one TMA load per tile, K by one TMA load per page (16 keys) through the block table;
-//   softmax        one thread per query row (= TMEM lane): its 128 scores in registers by tcgen05.ld, causal mask, online
-//                  maximum and sum, probabilities as bf16 back into TMEM over the scores;
-//   O += P V       A = P from TMEM, N = 128 head dims, K = 128 keys; V arrives by TMA exactly as the pages hold it,
-//                  [key][dim], and is used as an MN-major B operand (the dimension is the contiguous one): no transpose.
-// O stays in TMEM.  A row's scores are taken relative to a reference that follows its maximum only when that has grown by
-// more than 2^8 (the sum and O share the reference, so the quotient is the same; fp32 has the room, and bf16 probabilities
-// are relative): after the first blocks hardly any row rescales its 128 outputs.
+//   softmax        one thread per query row (= TMEM lane): its 128 scores by tcgen05.ld, twice -- causal mask and maximum, then
+//                  probabilities as bf16 back into TMEM over the scores, and their sum;
+//   P V            A = P from TMEM, N = 128 head dims, K = 128 keys; V arrives by TMA exactly as the pages hold it,
+//                  [key][dim], and is used as an MN-major B operand (the dimension is the contiguous one): no transpose;
+//   O = O * exp2(m_old - m_new) + P V    in registers (128 fp32 per thread), while the tensor pipe is at the next S.
+// Scores are taken relative to the exact running maximum, so that the largest probability of a row is 1, which bf16 holds
+// exactly.  (A reference that lags behind the maximum, with O summed up in TMEM, is 5 % faster -- 354 us against 374 for 2 x 4096
+// rows -- but rounds dominating probabilities, which the sum does not see: 2 to 3.5 x the error for peaked rows.)
 //
 // What bounds it: the softmax -- 16384 exponentials per block are 1024 cycles of an SM, the two MMAs are 1024 cycles of
-// tensor pipe -- and the chain S -> softmax -> P V of a CTA.  Two CTAs share an SM (96 KB of shared memory and 256 TMEM
-// columns each) and fill each other's gaps; a CTA's own copies are off the chain: K of the next block is fetched from the
-// moment S = Q K^T has read it, V from the moment P V has.  CTAs of late tiles (most keys) start first.
-// Measured (32 heads of 128, keys and values dense, CUDA events), one buffer of K / V and O in registers -> this:
-// 2 x 4096 rows 590 -> 354 us (777 TFLOP/s), 16 x 512 148 -> 104, 64 x 128 97 -> 74, 1 x 8192 1085 -> 639 (860); from pages
-// 358 us where they lie in order (eight per copy), 435 shuffled.
+// tensor pipe -- and the chain S -> softmax -> P V of a CTA.  Two CTAs share an SM (96 KB of shared memory, 256 TMEM
+// columns and 168 registers per thread each) and fill each other's gaps; a CTA's own copies are off the chain: K of the next
+// block is fetched from the moment S = Q K^T has read it, V from the moment P V has.  Scores and P V come 16 columns at a
+// time, the next 16 on their way while one is at work (32 at a time, each waited for: 681 us instead of 362 at 2 x 4096).
+// CTAs of late tiles (most keys) start first.
+// Measured (32 heads of 128, keys and values dense, CUDA events), one buffer of K / V and P through shared memory -> this:
+// 2 x 4096 rows 589 -> 374 us (735 TFLOP/s), 16 x 512 148 -> 109, 64 x 128 95 -> 75, 1 x 8192 1085 -> 672 (818); from pages,
+// 2 x 4096: 362 us where they lie in order (eight per copy), 418 shuffled.
 // Every wait is bounded; a CTA that gives up writes zeros.
 #include <math.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "tc_ptx.cuh"
@@ -79,8 +83,8 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
   uint8_t* sv = sk + NK * kSub;  // V block   [128 keys][128 d]   as two d-halves, exactly as the pages hold it
   __shared__ uint64_t kbar, vbar;  // a block's K (the first: and Q) / V has landed
   __shared__ uint64_t sbar;        // S = Q K^T has retired, and every P V before it
-  __shared__ uint64_t pbar;        // the four softmax warps have written P (and rescaled O)
-  __shared__ uint64_t obar, dbar;  // P V has retired / the last one has
+  __shared__ uint64_t pbar;        // the four softmax warps have written P, and taken the P V before into O
+  __shared__ uint64_t obar;        // P V has retired
   __shared__ uint32_t tmem_slot;
   __shared__ int s_abort;
 
@@ -104,7 +108,6 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
     mbar_init(&sbar, 1);
     mbar_init(&pbar, 4);
     mbar_init(&obar, 1);
-    mbar_init(&dbar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_k);
@@ -204,9 +207,8 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
 #pragma unroll
         for (int k = 0; k < kTile / 16; ++k)
           umma_bf16_ta(tmem_o, tmem_base + k * 8, make_smem_desc_mn(smem_u32(sv + k * 2048), kSub, 1024), idesc_pv,
-                       (kb > 0 || k > 0) ? 1u : 0u);
+                       k > 0 ? 1u : 0u);
         umma_commit(&obar);
-        if (kb + 1 == n_blocks) umma_commit(&dbar);
       }
       __syncwarp();
     }
@@ -218,8 +220,11 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
     const int q_lo = q_pos - q_pos % chunk;  // first key it sees
     const float scale = a.scale * kLog2e;
     const uint32_t lanes = (uint32_t)(warp * 32) << 16;
-    // reference of the row's scores, and their sum relative to it (a sink: a score of its own without a value)
-    float m_ref = a.sink ? a.sink[h] * kLog2e : -INFINITY, l_run = a.sink ? 1.f : 0.f;
+    // maximum of the row's scores so far, and their sum relative to it (a sink: a score of its own without a value)
+    float o[kDv];
+#pragma unroll
+    for (int i = 0; i < kDv; ++i) o[i] = 0.f;
+    float m_run = a.sink ? a.sink[h] * kLog2e : -INFINITY, l_run = a.sink ? 1.f : 0.f;
     bool ok = true;
     for (int kb = 0; kb < n_blocks && ok; ++kb) {
       const uint32_t par = kb & 1;
@@ -227,58 +232,64 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
       ok = __all_sync(0xffffffffu, mbar_wait(&sbar, par, &s_abort));
       if (!ok) break;
       tc_fence_after();
-      float s[kTile];
-#pragma unroll
-      for (int c0 = 0; c0 < kTile; c0 += 32) tmem_ld32_issue(tmem_base + lanes + c0, s + c0);
-      tmem_wait_ld();
       // Only the blocks on or past the diagonal need the causal / length mask, and those before the last row's chunk the
       // chunk's (uniform per CTA): every row of the tile sees every key of the blocks between.
       const bool need_mask = kstart + kTile - 1 > pos0 || kstart < lo_last;
-      if (need_mask) {
-        const int hi = min(q_pos, n_keys - 1) - kstart, lo = q_lo - kstart;
+      const int hi = min(q_pos, n_keys - 1) - kstart, lo = q_lo - kstart;  // keys of the block that this row sees
+      const uint32_t s_addr = tmem_base + lanes;
+      float buf[2][16];  // 16 scores at work, the next 16 on their way
+      // pass 1: row maximum (of the raw scores: the scale is positive)
+      float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      auto maximum = [&](auto masked) {
+        tmem_ld16_issue(s_addr, buf[0]);
 #pragma unroll
-        for (int i = 0; i < kTile; ++i)
-          if (i > hi || i < lo) s[i] = -INFINITY;
-      }
-      // row maximum (of the raw scores: the scale is positive)
-      float mx[4] = {s[0], s[1], s[2], s[3]};
+        for (int c = 0; c < kTile / 16; ++c) {
+          tmem_wait_ld16(buf[c & 1]);
+          if (c + 1 < kTile / 16) tmem_ld16_issue(s_addr + (c + 1) * 16, buf[(c + 1) & 1]);
 #pragma unroll
-      for (int i = 4; i < kTile; ++i) mx[i & 3] = fmaxf(mx[i & 3], s[i]);
-      const float m_blk = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale;
-      // a new reference: at the first visible key, and when the maximum has outgrown the old one
-      const bool grow = kb == 0 ? m_blk > m_ref : m_blk > m_ref + 8.f;
-      if (__any_sync(0xffffffffu, grow)) {
-        const float corr = grow ? (m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - m_blk)) : 1.f;
-        if (grow) m_ref = m_blk;
-        l_run *= corr;
-        if (kb > 0) {  // (every P V so far has retired: sbar)
-#pragma unroll 1
-          for (int c0 = 0; c0 < kDv; c0 += 32) {
-            float o[32];
-            tmem_ld32(tmem_o + lanes + c0, o);
+          for (int i = 0; i < 16; ++i)
+            if (!masked() || (c * 16 + i <= hi && c * 16 + i >= lo)) mx[i & 3] = fmaxf(mx[i & 3], buf[c & 1][i]);
+        }
+      };
+      if (need_mask)
+        maximum(std::true_type{});
+      else
+        maximum(std::false_type{});
+      const float m_new = fmaxf(m_run, fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * scale);
+      const float corr = m_run == -INFINITY ? 0.f : fast_exp2(m_run - m_new);  // (m_new == -inf: nothing seen yet, l and o are 0)
+      const float neg_m = m_new == -INFINITY ? 0.f : -m_new;                   // (then every key of the block is masked)
+      // pass 2: probabilities -> P (bf16 pairs, over scores that have been read), row sum
+      float sum = 0.f;
+      auto probabilities = [&](auto masked) {
+        tmem_ld16_issue(s_addr, buf[0]);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] *= corr;
-            tmem_st<32>(tmem_o + lanes + c0, o);
+        for (int c = 0; c < kTile / 16; ++c) {
+          tmem_wait_ld16(buf[c & 1]);
+          if (c + 1 < kTile / 16) tmem_ld16_issue(s_addr + (c + 1) * 16, buf[(c + 1) & 1]);
+          uint32_t pk[8];
+#pragma unroll
+          for (int i = 0; i < 16; i += 2) {
+            float p[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int key = c * 16 + i + e;
+              p[e] = fast_exp2(fmaf(buf[c & 1][i + e], scale, neg_m));
+              if (masked() && !(key <= hi && key >= lo)) p[e] = 0.f;
+              sum += p[e];
+            }
+            const __nv_bfloat162 b = __floats2bfloat162_rn(p[0], p[1]);
+            pk[i / 2] = *reinterpret_cast<const uint32_t*>(&b);
           }
+          tmem_st8_issue(s_addr + c * 8, pk);
         }
-      }
-      const float neg_m = m_ref == -INFINITY ? 0.f : -m_ref;  // (then every key so far is masked: probabilities are 0)
-      // probabilities -> P (bf16 pairs), row sum
-      float sum[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int c0 = 0; c0 < kTile; c0 += 64) {
-        float pk[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          const float p0 = fast_exp2(fmaf(s[c0 + 2 * i], scale, neg_m)), p1 = fast_exp2(fmaf(s[c0 + 2 * i + 1], scale, neg_m));
-          sum[(2 * i) & 3] += p0;
-          sum[(2 * i + 1) & 3] += p1;
-          const __nv_bfloat162 b = __floats2bfloat162_rn(p0, p1);
-          pk[i] = __uint_as_float(*reinterpret_cast<const uint32_t*>(&b));
-        }
-        tmem_st<32>(tmem_base + lanes + c0 / 2, pk);
-      }
-      l_run += (sum[0] + sum[1]) + (sum[2] + sum[3]);
+        tmem_wait_st();
+      };
+      if (need_mask)
+        probabilities(std::true_type{});
+      else
+        probabilities(std::false_type{});
+      l_run = fmaf(l_run, corr, sum);
+      m_run = m_new;
       if (n_keys - kstart < kTile) {
         // Last block, not full: the V rows of keys that do not exist (the tail of the last page, whatever the cache holds
         // there, and the pages that were not loaded) are zeroed once the copies have landed -- their probabilities are 0,
@@ -296,27 +307,32 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&pbar);
+      // O = O * corr + P V, while the tensor pipe is at the next block's scores
+      ok = __all_sync(0xffffffffu, mbar_wait(&obar, par, &s_abort));
+      if (!ok) break;
+      tc_fence_after();
+      tmem_ld16_issue(tmem_o + lanes, buf[0]);
+#pragma unroll
+      for (int c = 0; c < kDv / 16; ++c) {
+        tmem_wait_ld16(buf[c & 1]);
+        if (c + 1 < kDv / 16) tmem_ld16_issue(tmem_o + lanes + (c + 1) * 16, buf[(c + 1) & 1]);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) o[c * 16 + i] = fmaf(o[c * 16 + i], corr, buf[c & 1][i]);
+      }
     }
-    ok = ok && __all_sync(0xffffffffu, mbar_wait(&dbar, 0, &s_abort));
     if (!ok) s_abort = 1;
-    tc_fence_after();
     // ---- write ----------------------------------------------------------------------------------------------------------
     float inv = (ok && l_run > 0.f) ? 1.f / l_run : 0.f;
     if constexpr (!PAGED)
       if (a.gate && tid < rows) inv /= 1.f + __expf(-__bfloat162float(a.gate[(size_t)(row0 + tid) * a.ld_gate + h]));
     uint4* dst = reinterpret_cast<uint4*>(a.out + (size_t)(row0 + tid) * a.ld_out + (size_t)h * kDv);
+    if (tid < rows) {
 #pragma unroll
-    for (int c0 = 0; c0 < kDv; c0 += 32) {
-      float o[32];
-      tmem_ld32(tmem_o + lanes + c0, o);
-      if (tid < rows) {
+      for (int c = 0; c < kDv / 8; ++c) {
+        float f[8];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          float f[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) f[i] = ok ? o[c * 8 + i] * inv : 0.f;
-          dst[c0 / 8 + c] = pack8(f);
-        }
+        for (int i = 0; i < 8; ++i) f[i] = o[c * 8 + i] * inv;
+        dst[c] = pack8(f);
       }
     }
     if (!ok && tid == 0 && a.status) atomicOr(a.status, 1);

@@ -1,4 +1,4 @@
-"""Prompt attention whose running maximum moves: the reference of a row's scores follows it only past a factor of 2^8.
+"""Prompt attention whose running maximum moves: a row's sum and output are rescaled at every block that raises it.
 
 Values lie in [0.5, 1.5], so nothing cancels: probabilities rounded to bf16 (8 significant bits: 2^-8 relative at most), the
 result rounded to bf16 (2^-8) and fp32 sums in between bound every output's relative error by 2^-7.
@@ -11,8 +11,8 @@ from conftest import load
 pytestmark = pytest.mark.gpu
 
 
-# growth of the scores per key, in powers of two of a probability: none, within the factor over blocks, past it at some
-# blocks and rows only, past it everywhere, falling
+# growth of the scores per key, in powers of two of a probability: none, little over a block, 2^9 over a block, past what fp32
+# holds, falling
 @pytest.mark.parametrize("growth", [0.0, 0.01, 0.07, 0.5, -0.05])
 @pytest.mark.parametrize("lens", [[1], [127, 128, 129], [700], [64, 513]])
 @pytest.mark.parametrize("Dk,Dv", [(128, 128), (64, 128), (128, 64)])
@@ -44,6 +44,29 @@ def test_scores_that_grow(growth, lens, Dk, Dv):
         got = out[base:base + n].double()
         assert ((got - want).abs() / want).max().item() < 2.0 ** -7
         base += n
+
+
+# Two keys share a row's probability, the later one with the larger score, and only that one has a value: its probability is 1,
+# which bf16 holds exactly, the sum is fp32, so the output is the 64-bit value rounded once: off by half a unit of its last of 8
+# bits, plus 2^-18 for exponential, sum and quotient in fp32.  (A reference that lags behind the maximum would round the
+# probability a second time.)
+@pytest.mark.parametrize("late", [131, 200, 300])
+def test_the_largest_probability_is_exact(late):
+    ops = load("ops")
+    H, D, T = 24, 64, 384
+    g = torch.Generator(device="cuda").manual_seed(late)
+    q, k, v = (torch.zeros(T, H, D, device="cuda") for _ in range(3))
+    q[:, :, 0], k[:, :, 0] = 1.0, -64.0
+    growth = torch.linspace(0.05, 5.5, H, device="cuda").bfloat16()
+    k[5, :, 0], k[late, :, 0] = 0.0, growth.float()
+    v[late] = torch.rand(H, D, generator=g, device="cuda") + 0.5
+    kv = torch.cat([k.flatten(1), v.flatten(1)], 1).bfloat16().contiguous()
+    tiles = torch.tensor([(0, o, 128, o) for o in range(0, T, 128)], dtype=torch.int32, device="cuda")
+    out = torch.zeros(T, H * D, device="cuda").bfloat16()
+    ops.prefill_attention_dense(q.flatten(1).bfloat16().contiguous(), kv, H * D, tiles, 3, H, D, D, 1.0, out)
+    want = v[late].bfloat16().double() / (1 + torch.exp(-growth.double()))[:, None]
+    got = out.view(T, H, D)[late:].double()
+    assert ((got - want).abs() <= 2.0 ** (want.log2().floor() - 8) + want * 2.0 ** -18).all()
 
 
 # pages of a sequence one after the other in the pool are fetched eight at a time: the same bytes as page by page
