@@ -57,6 +57,10 @@ extern "C" {
                                (gate/up/down when only q/k/v/o carry adapters): run the kernel variant the LoRA
                                calls use, so one code footprint stays hot in the instruction caches for the whole
                                step; results are identical either way */
+#define MLORA_STABLE_SUMS 1024 /* sums over `in` as the one-CTA plan (mlora_linear_plan) takes them, bit for bit: pairs of
+                               CTAs only where that plan has whole tiles, whose sums are the same.  For projections in
+                               front of a discrete choice (an expert router picks the largest of its scores): there
+                               another order of fp32 sums is another choice at a near tie */
 
 int mlora_version(void);
 const char* mlora_last_error(void);
@@ -146,6 +150,13 @@ size_t mlora_linear_workspace(int32_t T, int32_t in, int32_t out);
  * row tiles c / [6] + s * [7], s = 0 .. [8] - 1; 0 with [6] > 0: contiguous chunks of [8] tiles per group), [8] steps per
  * group, [9] groups, [10] chunk length in the last, narrower group (chunk form), [11] 0. */
 int mlora_linear_plan(int32_t T, int32_t in, int32_t out, int32_t* h_plan12);
+/* ... and whether a call runs on pairs of CTAs instead, and how (host side only as well).  r_max 0: no adapters; n_mod,
+ * h_mod_offsets and flags as for mlora_linear.  h_plan6 (HOST, 6 int32): [0] token rows per tile (0: the call stays on the
+ * one-CTA kernel, the rest is 0 too), [1] pairs launched, [2] row tiles (128 outputs), [3] token tiles, [4] pairs of row tiles
+ * (a module with an odd number of row tiles ends in a pair of one), [5] token tiles per group: within a group of token tiles
+ * pair w takes (row pair, token tile) number w, w + [1], ..., row pair major. */
+int mlora_linear_pair_plan(int32_t T, int32_t in, int32_t out, int32_t r_max, int32_t n_mod, const int32_t* h_mod_offsets,
+                           int32_t flags, int32_t* h_plan6);
 /* The same for a call with these flags: more than mlora_linear_workspace only for MLORA_SILU_MUL | MLORA_LORA_PER_ROW. */
 size_t mlora_linear_workspace_flags(int32_t T, int32_t in, int32_t out, int32_t flags);
 /* Weight pre-packing (load time).  Rewrites W [out,in] bf16 as tiles [ceil(out/128)][ceil(in/64)] of

@@ -13,6 +13,25 @@ extern "C" int mlora_linear_plan(int32_t T, int32_t in, int32_t out, int32_t* h_
   return MLORA_OK;
 }
 
+extern "C" int mlora_linear_pair_plan(int32_t T, int32_t in, int32_t out, int32_t r_max, int32_t n_mod,
+                                      const int32_t* h_mod_offsets, int32_t flags, int32_t* h_plan6) {
+  MLORA_REQUIRE(T > 0 && in > 0 && out > 0 && r_max >= 0 && n_mod >= 1 && n_mod <= 8 && (n_mod == 1 || h_mod_offsets) && h_plan6,
+                "linear_pair_plan: bad arguments");
+  LinearArgs a{};
+  a.T = T;
+  a.in = in;
+  a.out = out;
+  a.flags = flags;
+  a.r_max = r_max;
+  static const float some = 0.f;  // (only whether there are shrink outputs counts)
+  a.u = r_max ? &some : nullptr;
+  a.n_mod = n_mod;
+  for (int m = 0; m <= n_mod && n_mod > 1; ++m) a.mod_off[m] = h_mod_offsets[m];
+  for (int i = 0; i < 6; ++i) h_plan6[i] = 0;
+  if (linear_pair_chosen(a)) linear_pair_plan(a, h_plan6);
+  return MLORA_OK;
+}
+
 static size_t pre_offset(int32_t T, int32_t in, int32_t out) { return (linear_tc_workspace(T, in, out) + 255) & ~(size_t)255; }
 
 extern "C" size_t mlora_linear_workspace_flags(int32_t T, int32_t in, int32_t out, int32_t flags) {

@@ -136,6 +136,8 @@ void linear_tc_plan(int T, int in, int out, int32_t* v12);
 int launch_linear_tc(const LinearArgs& a, void* work, size_t work_bytes, cudaStream_t st);
 // The same on pairs of CTAs, for prompt-size batches (of `work` only the status word).
 bool linear_pair_supported(const LinearArgs& a);
+bool linear_pair_chosen(const LinearArgs& a);
+void linear_pair_plan(const LinearArgs& a, int32_t* v6);
 int launch_linear_pair(const LinearArgs& a, void* work, cudaStream_t st);
 int launch_grouped_pair(const GroupedArgs& g, void* work, cudaStream_t st);
 // LoRA expand laid out by (row, output feature), added to y in place (batches with many distinct adapters).

@@ -704,6 +704,17 @@ bool linear_pair_supported(const LinearArgs& a) {
   return 4ll * ((a.T + 127) / 128) * pair_row_pairs(a) >= 3ll * (sm_count() / 2);
 }
 
+void linear_pair_plan(const LinearArgs& a, int32_t* v) {
+  const PairPlan pl = pair_plan(a.T, a.in, pair_row_pairs(a));
+  const long long tiles = (long long)pl.tok_tiles * pl.row_pairs;
+  v[0] = pl.bn;
+  v[1] = (int)(tiles < sm_count() / 2 ? tiles : sm_count() / 2);
+  v[2] = (a.out + BM - 1) / BM;
+  v[3] = pl.tok_tiles;
+  v[4] = pl.row_pairs;
+  v[5] = pl.gt;
+}
+
 int launch_linear_pair(const LinearArgs& a, void* work, cudaStream_t st) {
   PairParams p{};
   p.a = a;

@@ -209,7 +209,7 @@ int launch(const LinearArgs& a, const Plan& pl, void* work, cudaStream_t st) {
   }
   if constexpr (BN == 256) {
     // Everything else of this size runs on pairs of CTAs: enough whole 256-token tiles for this plan are more than enough for
-    // linear_pair_supported(), which leaves only the expand on CUDA cores.
+    // linear_pair_chosen(), which leaves only the expand on CUDA cores.
     if (p.lora_mode != 1) return fail(MLORA_EINVAL, "linear: no one-CTA kernel for 256-token tiles without a CUDA-core expand");
     launch_pdl_if(pdl_enabled_gemm(), linear_tc_kernel<BN, 1>, pl.grid, kThreads, C::kSmemBytes, st, mw, mx, mb, my, p);
   } else {
@@ -326,10 +326,20 @@ size_t linear_tc_workspace(int T, int in, int out) {
   return kHeaderBytes + kMaxGrid * 4 + (size_t)kMaxGrid * 2 * bn * BM * sizeof(float);
 }
 
+// Whole tiles are summed k-block after k-block by both kernels; split tiles are summed in parts.  Calls that ask for the plan's
+// sums (MLORA_STABLE_SUMS) give up pairs where the plan splits: 129 to some 3000 rows of a 4096-wide projection, 1024 rows
+// 4096 -> 4096 67 us instead of 41.
+bool linear_pair_chosen(const LinearArgs& a) {
+  if (!linear_pair_supported(a)) return false;
+  if (!(a.flags & MLORA_STABLE_SUMS)) return true;
+  const Plan pl = make_plan(a.T, a.in, a.out);
+  return pl.wave_gt > 0 || pl.per_cta % pl.k_blocks == 0;
+}
+
 int launch_linear_tc(const LinearArgs& a, void* work, size_t work_bytes, cudaStream_t st) {
   const size_t need = linear_tc_workspace(a.T, a.in, a.out);
   if (work_bytes < need) return fail(MLORA_ESIZE, "linear: workspace of %zu bytes needed, %zu given", need, work_bytes);
-  if (linear_pair_supported(a)) return launch_linear_pair(a, work, st);
+  if (linear_pair_chosen(a)) return launch_linear_pair(a, work, st);
   Plan pl = make_plan(a.T, a.in, a.out);
   switch (pl.bn) {
     case 16: return launch<16>(a, pl, work, st);

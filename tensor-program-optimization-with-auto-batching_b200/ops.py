@@ -14,6 +14,7 @@ from . import _lib
 from ._lib import check
 
 OUT_F32, SILU_MUL, FORCE_SIMT, W_PACKED, B_PACKED, SHARE_LORA_KERNEL, LORA_PER_ROW, B_SPLIT = 1, 2, 4, 8, 16, 32, 64, 128
+STABLE_SUMS = 1024
 
 
 def _ptr(t):  # (plain numbers: the prototypes convert them)

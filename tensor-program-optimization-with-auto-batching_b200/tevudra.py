@@ -245,6 +245,11 @@ class TevudraEngine(PlainEngine):
         self._n_tiles = 0
 
     # -- pieces of a layer ----------------------------------------------------------------------------------------
+    def _linear(self, x, W, out, flags=0):
+        # what stands in front of an expert router keeps its order of sums whatever kernel is fastest: another rounding picks
+        # another expert wherever two scores are nearly the same
+        return super()._linear(x, W, out, flags if self.m.dtype == torch.float32 else flags | ops.STABLE_SUMS)
+
     def _grouped(self, x, W, out, flags=0, **kw):
         if self.m.dtype == torch.float32:
             flags &= ~OUT_F32

@@ -98,3 +98,18 @@ def test_grouped(T, K, N, groups):
     ref = torch.cat([x[:, i * K:(i + 1) * K].float() @ W[i].float().t() * torch.sigmoid(gate[:, i:i + 1].float()) for i in range(groups)], 1)
     assert ops.status_word(work) == 0
     assert _err(y, ref) < TOL
+
+
+# the same sums as the one-CTA kernel, bit for bit, where its plan has whole tiles (the last three) and where it splits them.  A
+# rank pitch of 24 keeps a call on that kernel; no row has an adapter.
+@pytest.mark.parametrize("T,K,N", [(300, 2048, 8192), (1000, 512, 4096), (2048, 8192, 2048), (3000, 4096, 4096), (1184, 256, 2048),
+                                   (5000, 128, 6144), (9473, 200, 136)])
+def test_stable_sums_are_those_of_the_one_cta_kernel(T, K, N):
+    ops = load("ops")
+    g, x, W, _ = _setup(T, K, N, T)
+    stack = ops.LoraStack(torch.zeros(1, 24, K, device="cuda").bfloat16(), torch.zeros(1, N, 24, device="cuda").bfloat16(),
+                          torch.full((1,), 24, dtype=torch.int32, device="cuda"), torch.ones(1, device="cuda"), 24, 1, (0, N))
+    slots = torch.full((T,), -1, dtype=torch.int32, device="cuda")
+    want = ops.linear(x, ops.PackedWeight(W), stack, slots, torch.zeros(T, 24, device="cuda"), flags=ops.OUT_F32)
+    got = ops.linear(x, ops.PackedWeight(W), flags=ops.OUT_F32 | ops.STABLE_SUMS)
+    assert torch.equal(got, want)

@@ -1,5 +1,6 @@
-"""Host-side planning of the tensor-core projection (``mlora_linear_plan``): whatever the shape, every tile -- or, at decode
-sizes, every k-block of every tile -- is dealt to exactly one CTA.  No GPU: the plan is arithmetic on the shape (the SM
+"""Host-side planning of the tensor-core projection (``mlora_linear_plan`` of the one-CTA kernel, ``mlora_linear_pair_plan``
+of pairs of CTAs): whatever the shape, every tile -- or, at decode sizes, every k-block of every tile -- is dealt to exactly one
+CTA or pair.  No GPU: the plan is arithmetic on the shape (the SM
 count falls back to a B200's 148 without a device)."""
 import ctypes as C
 
@@ -88,3 +89,55 @@ def test_prompt_passes_take_256_token_tiles_and_decode_sizes_do_not():
     assert _plan(16, 4096, 4096)["bn"] == 16
     p = _plan(8192, 4096, 12288)
     assert (p["gt"], p["lanes"], p["steps"], p["groups"]) == (16, 9, 11, 2)
+
+
+def _pair_plan(T, K, N, mods=None, rank=0, flags=0):
+    lib = load("_lib").lib()
+    v, offs = (C.c_int32 * 6)(), (C.c_int32 * len(mods))(*mods) if mods else None
+    assert lib.mlora_linear_pair_plan(T, K, N, rank, len(mods) - 1 if mods else 1, offs, flags, v) == 0
+    return dict(zip(("bn", "pairs", "row_tiles", "tok_tiles", "row_pairs", "gt"), list(v)))
+
+
+def _pair_rows(p, mods, row_pair):
+    """Row tiles of a row pair (the kernel's pair_rows, restated): never of two modules."""
+    first, end, m = 0, p["row_tiles"], 0
+    if len(mods) > 2:
+        while True:
+            first, end = mods[m] // 128, mods[m + 1] // 128 if m + 2 < len(mods) else p["row_tiles"]
+            n = (end - first + 1) // 2
+            if row_pair < n or m + 2 >= len(mods):
+                break
+            row_pair, m = row_pair - n, m + 1
+    return [t for t in (first + 2 * row_pair, first + 2 * row_pair + 1) if t < end], m
+
+
+@pytest.mark.parametrize("mods", [None, [0, 384, 640], [0, 128, 256, 1280], [0, 128, 384, 512, 896]])
+@pytest.mark.parametrize("T,K,N", SHAPES + [(129, 64, 20000), (333, 4096, 12288), (700, 16384, 9000), (9473, 64, 128), (70000, 16384, 264)])
+def test_pairs_compute_every_tile_exactly_once(T, K, N, mods):
+    mods = [0, N] if mods is None else mods + [N]
+    if mods[-2] >= N:
+        pytest.skip("fewer outputs than module offsets")
+    p = _pair_plan(T, K, N, mods, 16 if len(mods) > 2 else 0)
+    if p["bn"] == 0:
+        assert T <= 128 or 4 * -(-T // 128) * sum((-(-b // 128) - a // 128 + 1) // 2 for a, b in zip(mods, mods[1:])) < 3 * 74
+        return
+    assert p["bn"] % 32 == 0 and 64 <= p["bn"] <= 256 and p["tok_tiles"] == -(-T // p["bn"]) and p["row_tiles"] == -(-N // 128)
+    n_tiles = p["tok_tiles"] * p["row_pairs"]
+    assert p["pairs"] == min(n_tiles, 74) and p["gt"] >= 1
+    seen = []
+    for w in range(p["pairs"]):
+        for idx in range(w, n_tiles, p["pairs"]):  # the kernel's pair_tile, restated
+            grp, rem = divmod(idx, p["gt"] * p["row_pairs"])
+            width = min(p["gt"], p["tok_tiles"] - grp * p["gt"])
+            rows, m = _pair_rows(p, mods, rem // width)
+            assert rows and all(mods[m] <= t * 128 < mods[m + 1] for t in rows)
+            seen += [(t, grp * p["gt"] + rem % width) for t in rows]
+    assert sorted(seen) == [(r, t) for r in range(p["row_tiles"]) for t in range(p["tok_tiles"])]
+
+
+@pytest.mark.parametrize("T,K,N", SHAPES)
+def test_stable_sums_take_pairs_only_where_no_tile_is_split(T, K, N):
+    p = _plan(T, K, N)
+    whole = p["gt"] > 0 or p["per_cta"] % p["k_blocks"] == 0
+    stable = load("ops").STABLE_SUMS
+    assert (_pair_plan(T, K, N, flags=stable)["bn"] > 0) == (whole and _pair_plan(T, K, N)["bn"] > 0)
