@@ -292,6 +292,7 @@ __device__ __forceinline__ uint32_t cluster_rank() {
   return r;
 }
 __device__ __forceinline__ void cluster_sync() {
+  __syncwarp();  // (.aligned: the warp arrives as one, whatever its threads did before)
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
