@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(kShrinkThreads, 1) lora_shrink_tc_kernel(const
   const int stage_bytes = kXTile + ((nj_max * a_tile + 1023) & ~1023);
   const int stages = min(kMaxStages, p.ring_bytes / stage_bytes);
 
+  int issued = 0;  // stages the producer has requested
   if (warp == 0 && lane == 0) {
     // ---- producer: token tile + the pass's adapter tiles per k-block ----
     int g = 0;
@@ -145,14 +146,7 @@ __global__ void __launch_bounds__(kShrinkThreads, 1) lora_shrink_tc_kernel(const
           tma_load_2d(st + kXTile + j * a_tile, &map_a, kb * BK, s_list[j0 + j] * p.r_tot, &full_bar[s]);
       }
     }
-    if (!ok) {
-      // copies already issued still land in this CTA's shared memory: wait for them (bounded) before leaving
-      int dummy = 0;
-      for (int back = 1; back <= stages && back <= g; ++back) {
-        const int gi = g - back;
-        mbar_wait(&full_bar[gi % stages], (gi / stages) & 1, &dummy);
-      }
-    }
+    issued = g;
   } else if (warp == 1 && lane == 0) {
     // ---- MMA issuer ----
     const uint32_t idesc = make_idesc(kTok, p.n_pad);
@@ -232,11 +226,20 @@ __global__ void __launch_bounds__(kShrinkThreads, 1) lora_shrink_tc_kernel(const
     }
   }
   __syncthreads();
+  if (s_abort && tid == 0) {
+    // whoever gave up: copies already issued still land in this CTA's shared memory, wait for them (bounded) before leaving
+    int dummy = 0;
+    for (int back = 1; back <= stages && back <= issued; ++back) {
+      const int gi = issued - back;
+      mbar_wait(&full_bar[gi % stages], (gi / stages) & 1, &dummy);
+    }
+  }
   if (p.splits > 1) {
-    if (split && s_abort && warp >= 2)  // (a NaN in a share makes the row's sums NaN)
-      for (int c = 0; c < p.r_tot / 4; ++c) part[c * kTok + (warp & 3) * 32 + lane] = make_float4(NAN, NAN, NAN, NAN);
     cluster_sync();
     if (split) {
+      // one share missing: the rows are NaN.  (Told by a word outside the ring, where late copies of the CTA that failed may land.)
+      bool whole = true;
+      for (int q = 0; q < p.splits; ++q) whole = whole && ld_cluster(&s_abort, q) == 0;
       const int rows = kTok / p.splits, r0 = rank * rows;
       for (int i = tid; i < rows * (p.r_tot / 4); i += kShrinkThreads) {
         const int row = r0 + i % rows, c = i / rows, t = t0 + row;
@@ -244,6 +247,7 @@ __global__ void __launch_bounds__(kShrinkThreads, 1) lora_shrink_tc_kernel(const
         float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
         if (s_seg[row] >= 0)
           for (int q = 0; q < p.splits; ++q) {
+            if (!whole) sum.x = sum.y = sum.z = sum.w = NAN;
             const float4 v = ld_cluster4(&part[c * kTok + row], q);
             sum.x += v.x, sum.y += v.y, sum.z += v.z, sum.w += v.w;
           }

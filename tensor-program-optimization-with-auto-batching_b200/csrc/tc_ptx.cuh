@@ -296,7 +296,18 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Four floats at a shared-memory address of the CTA with this rank in the cluster.
+// A word / four floats at a shared-memory address of the CTA with this rank in the cluster.
+__device__ __forceinline__ int ld_cluster(const int* p, uint32_t rank) {
+  int v;
+  asm volatile(
+      "{\n\t.reg .u32 a;\n\t"
+      "mapa.shared::cluster.u32 a, %1, %2;\n\t"
+      "ld.shared::cluster.s32 %0, [a];\n\t}"
+      : "=r"(v)
+      : "r"(smem_u32(p)), "r"(rank)
+      : "memory");
+  return v;
+}
 __device__ __forceinline__ float4 ld_cluster4(const void* p, uint32_t rank) {
   float4 v;
   asm volatile(

@@ -21,3 +21,13 @@ def test_cluster_barriers_are_reached_by_whole_warps():
     for name in os.listdir(os.path.join(ROOT, PKG, "csrc")):
         if name != "tc_ptx.cuh":
             assert "barrier.cluster" not in _source(name)
+
+
+def test_a_failed_share_of_the_shrink_is_told_outside_the_ring():
+    """Copies still in flight may land on whatever a CTA that gave up writes into its ring; and whoever gave up, the CTA waits for
+    what the producer has requested."""
+    src = _source("shrink_tc.cu")
+    tail = src[src.index("__syncthreads();\n  if (s_abort && tid == 0)"):]
+    assert "part[" in tail and not re.search(r"part\[[^\]]*\]\s*=", tail)  # (read, not written)
+    first = tail.index("cluster_sync();")
+    assert tail.index("mbar_wait(&full_bar") < first < tail.index("ld_cluster(&s_abort") < tail.index("ld_cluster4(&part")
