@@ -310,8 +310,10 @@ int launch_lora_shrink_tc(const void* x, int64_t ldx, const void* A_all, const i
   }
   // as many CTAs per tile as the chip holds, down to eight k-blocks each
   const int tiles = (T + kTok - 1) / kTok;
+  int sms = 148;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   p.splits = 1;
-  while (p.splits < 8 && tiles * p.splits * 2 <= 148 && p.k_blocks >= p.splits * 16) p.splits *= 2;
+  while (p.splits < 8 && tiles * p.splits * 2 <= sms && p.k_blocks >= p.splits * 16) p.splits *= 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(tiles, p.splits);
   cfg.blockDim = dim3(kShrinkThreads);

@@ -9,9 +9,9 @@ from conftest import load
 pytestmark = pytest.mark.gpu
 
 
-# tiles of 128 rows: 2 (ragged), 9, 19 and 37 are the last that eight, four and two CTAs share, 75 one CTA each; in: fewer
-# k-blocks than two CTAs take, a count that does not divide, a ragged last block
-@pytest.mark.parametrize("T", [256, 257, 1152, 1153, 2432, 4736, 9500])
+# tiles of 128 rows: 2 (whole, ragged); 18 | 19, 37 | 38 and 74 | 75 are where eight, four and two CTAs last share one and
+# fewer do (148 SMs); in: fewer k-blocks than two CTAs take, a count that does not divide, a ragged last block
+@pytest.mark.parametrize("T", [256, 257, 1152, 1153, 2304, 2305, 2432, 4736, 4737, 9472, 9473, 9500])
 @pytest.mark.parametrize("K", [64, 1000, 4104])
 @pytest.mark.parametrize("rank,n_mod,adapters,layout", [(16, 3, 2, "runs"), (64, 1, 1, "runs"), (8, 1, 40, "mixed"), (64, 3, 3, "mixed"), (16, 1, 5, "none")])
 def test_against_fp64(T, K, rank, n_mod, adapters, layout):
