@@ -20,7 +20,8 @@
 // of those operands to shared memory while the tile's own MMAs run (they have that long; done by the output warps, between two
 // tiles, it held the tensor pipe up).  The room holds a number of adapters at a time ("batch").
 //
-// Every wait is bounded; on expiry the CTA records a code in the status word, stops issuing work and goes to the teardown,
+// Every wait on an mbarrier is bounded, and the warps of a role that meet at a named barrier leave together or not at all
+// (bar_all); on expiry the CTA records a code in the status word, stops issuing work and goes to the teardown,
 // where the pair meets before either CTA leaves or frees its TMEM.
 #include <atomic>
 
@@ -409,8 +410,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(LORA), 
         grp = gt.group;
         y_col = gt.group * p.g.y_cols;
       }
-      const bool got = mbar_wait_pair(&acc_full[buf], (j >> 1) & 1, &s_abort);
-      if (!__all_sync(0xffffffffu, got)) {
+      if (!bar_all(1, mbar_wait_pair(&acc_full[buf], (j >> 1) & 1, &s_abort))) {
         if (!s_abort) {
           s_abort = 1;
           atomicOr(p.status, 4);
@@ -501,7 +501,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(LORA), 
       __syncwarp();
       asm volatile("bar.sync 2, 128;" ::: "memory");
     };
-    // one lane waits for its warp, so that the warp stays converged
+    // one lane waits for its warp; the four warps go on, or give up, together
     auto wait = [&](uint64_t* b, uint32_t parity) {
       int w = 1;
       if (lane == 0) w = mbar_wait_pair(b, parity, &s_abort) ? 1 : 0;
@@ -510,7 +510,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(LORA), 
         s_abort = 1;
         atomicOr(p.status, 32);
       }
-      return w != 0;
+      return bar_all(2, w != 0);
     };
     for (int idx = worker; idx < n_tiles && ok; idx += workers, ++j) {
       const PairTile pt = pair_tile(p, idx, tok_tiles);

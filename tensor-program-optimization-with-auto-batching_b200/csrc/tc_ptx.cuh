@@ -161,6 +161,21 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void epi_bar_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// One verdict for the 128 threads of a role that meet at barrier `id`: true if all of them say so.  After a wait that may have run
+// out in some warps only; a warp that left by itself would keep the others at their next barrier for good.
+__device__ __forceinline__ bool bar_all(int id, bool ok) {
+  uint32_t r;
+  __syncwarp();
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.and.aligned.pred q, %2, 128, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"((uint32_t)ok), "r"(id)
+      : "memory");
+  return r != 0;
+}
 
 // 32 lanes x 32 columns of fp32: register i of lane l = TMEM[lane_base + l][col + i].
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {

@@ -31,3 +31,17 @@ def test_a_failed_share_of_the_shrink_is_told_outside_the_ring():
     assert "part[" in tail and not re.search(r"part\[[^\]]*\]\s*=", tail)  # (read, not written)
     first = tail.index("cluster_sync();")
     assert tail.index("mbar_wait(&full_bar") < first < tail.index("ld_cluster(&s_abort") < tail.index("ld_cluster4(&part")
+
+
+@pytest.mark.parametrize("name", ["linear_pair_tc.cu"])
+def test_output_warps_share_a_verdict(name):
+    """A warp that leaves by itself after a wait that ran out keeps the others at their next named barrier for good."""
+    waits = re.findall(r"^.*mbar_wait\w*\(&acc_full.*$", _source(name), flags=re.M)
+    assert waits and all("bar_all(1, mbar_wait" in w for w in waits), waits
+
+
+def test_operand_builders_of_a_pair_share_a_verdict():
+    src = _source("linear_pair_tc.cu")
+    role = src[src.index("const uint32_t cache_lead"):src.index("__syncthreads();\n  if (s_abort)")]
+    assert role.count("mbar_wait_pair(") == 1  # in `wait` alone, which returns the role's verdict
+    assert "return bar_all(2, w != 0);" in role
