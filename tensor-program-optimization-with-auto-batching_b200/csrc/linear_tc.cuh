@@ -1306,7 +1306,7 @@ __global__ void __launch_bounds__(kThreads, 1) linear_tc_kernel(const __grid_con
         }
       }
 
-      if (!mbar_wait(&acc_full[buf], (j >> 1) & 1, &s_abort)) {
+      if (!bar_all(1, mbar_wait(&acc_full[buf], (j >> 1) & 1, &s_abort))) {
         if (!s_abort) {
           s_abort = 1;
           atomicOr(p.status, 4);

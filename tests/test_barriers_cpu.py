@@ -33,7 +33,7 @@ def test_a_failed_share_of_the_shrink_is_told_outside_the_ring():
     assert tail.index("mbar_wait(&full_bar") < first < tail.index("ld_cluster(&s_abort") < tail.index("ld_cluster4(&part")
 
 
-@pytest.mark.parametrize("name", ["linear_pair_tc.cu"])
+@pytest.mark.parametrize("name", ["linear_pair_tc.cu", "linear_tc.cuh", "chain_tc.cu"])
 def test_output_warps_share_a_verdict(name):
     """A warp that leaves by itself after a wait that ran out keeps the others at their next named barrier for good."""
     waits = re.findall(r"^.*mbar_wait\w*\(&acc_full.*$", _source(name), flags=re.M)
