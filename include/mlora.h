@@ -323,7 +323,7 @@ int mlora_paged_attention(const void* d_qkv, int64_t ld, void* d_k_pages, void* 
 /* mlora_prefill_attention: causal attention for prompt rows on the tensor cores, after mlora_kv_append_rope has
  * rotated q in place and stored the rows' k / v -- the ragged prefill path of attention_with_fused_qkv
  * (tvm/llama_auto_batcher/llama_for_causal_lm.py:55-64; prefill call llama_exec_graph.py:75-85).  The rows are given as
- * tiles: d_tiles [n_tiles][4] int32 = (cache slot, index of the tile's first row in d_qkv / d_out, rows <= 128,
+ * tiles: d_tiles [n_tiles][4] int32 = (cache slot, index of the tile's first row in d_qkv / d_out, rows <= 128; without rows: a no-op,
  * position of that first row in its sequence); the rows of a tile are consecutive rows of ONE sequence at consecutive
  * positions.  Same result as mlora_paged_attention(fused_append = 0) on those rows (different summation order).
  * head_dim 128 and page size 16 only; n_pages_total = pages in d_k_pages / d_v_pages; T = rows of d_qkv.

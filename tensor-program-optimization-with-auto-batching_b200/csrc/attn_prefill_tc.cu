@@ -92,6 +92,7 @@ __global__ void __launch_bounds__(kPfThreads, 2) prefill_attn_tc_kernel(const __
   const int tile = a.n_tiles - 1 - (int)(blockIdx.x / a.Hq), h = blockIdx.x % a.Hq;
   const int rep = a.Hq / a.Hkv, kvh = h / rep;
   const int slot = a.tiles[tile * 4 + 0], row0 = a.tiles[tile * 4 + 1], rows = a.tiles[tile * 4 + 2], pos0 = a.tiles[tile * 4 + 3];
+  if (rows <= 0) return;  // (the whole CTA, before it has asked for anything)
   const int32_t* bt = PAGED ? a.block_table + (size_t)slot * a.max_pages : nullptr;
   constexpr int kDv = NV * 64;
   const int chunk = a.chunk > 0 ? a.chunk : 0x7fffffff;

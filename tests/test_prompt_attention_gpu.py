@@ -69,6 +69,28 @@ def test_the_largest_probability_is_exact(late):
     assert ((got - want).abs() <= 2.0 ** (want.log2().floor() - 8) + want * 2.0 ** -18).all()
 
 
+# tiles without rows, at position 0 and further on, in front of, between and behind others: nothing happens, nothing is reported
+@pytest.mark.parametrize("paged", [False, True])
+def test_tiles_without_rows(paged):
+    ops = load("ops")
+    H, D, n = 2, 64, 200
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q, kv = torch.randn(n, H * D, generator=g, device="cuda").bfloat16(), torch.randn(208, 2 * H * D, generator=g, device="cuda").bfloat16()
+    k, v = (t.reshape(13, 16, H, D).transpose(1, 2).contiguous() for t in (kv[:, :H * D], kv[:, H * D:]))
+    table = torch.arange(13, dtype=torch.int32, device="cuda")[None]
+    outs = []
+    for tiles in ([(0, 0, 128, 0), (0, 128, 72, 128)], [(0, 0, 0, 0), (0, 0, 128, 0), (0, 128, 0, 128), (0, 128, 72, 128), (0, 0, 0, 0), (0, 0, -5, 0)]):
+        t = torch.tensor(tiles, dtype=torch.int32, device="cuda")
+        out, status = torch.full((n, H * D), 7.0, device="cuda").bfloat16(), torch.zeros(1, dtype=torch.int32, device="cuda")
+        if paged:
+            ops.prefill_attention_masked(q, k, v, table, t, len(tiles), H, D ** -0.5, out, status=status)
+        else:
+            ops.prefill_attention_dense(q, kv, H * D, t, len(tiles), H, D, D, D ** -0.5, out, status=status)
+        assert int(status) == 0
+        outs.append(out)
+    assert torch.equal(*outs)
+
+
 # pages of a sequence one after the other in the pool are fetched eight at a time: the same bytes as page by page
 @pytest.mark.parametrize("n", [1, 112, 128, 129, 640, 1000])
 @pytest.mark.parametrize("D,Hq,Hkv", [(128, 4, 2), (64, 3, 3)])
