@@ -127,16 +127,18 @@ class PagedCache:
         """:meth:`begin_forward` for a caller that uploads the rows with others of its own: two int32 arrays on the host."""
         seq_ids = [int(s) for s in seq_ids]
         append_lens = [int(a) for a in append_lens]
-        slots = np.array([self._slot_of[s] for s in seq_ids], dtype=np.int32)
-        lens = np.array(append_lens, dtype=np.int64)
+        both = list(zip(seq_ids, append_lens))  # (what one of them has more of has no rows)
+        slots = np.array([self._slot_of[s] for s, _ in both], dtype=np.int32)
+        lens = np.array([a for _, a in both], dtype=np.int64)
         first = self._len_host[slots]
         changed = []
         try:
-            for sid, n in zip(seq_ids, (first + lens).tolist()):
+            for (sid, _), n in zip(both, (first + lens).tolist()):
                 changed += self._take_pages(sid, n)
         finally:  # (sequences before one that finds no page keep what they got)
             self._push_pages(changed)
         self._pending = (seq_ids, append_lens)
+        lens = np.maximum(lens, 0)  # a negative length takes tokens back at the end of the forward
         start = first.astype(np.int64) - (np.cumsum(lens) - lens)  # position of a sequence's row r = start + r
         return np.repeat(slots, lens), (np.arange(int(lens.sum())) + np.repeat(start, lens)).astype(np.int32)
 
