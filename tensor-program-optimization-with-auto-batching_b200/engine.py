@@ -123,6 +123,7 @@ class EngineBase:
             T = sum(n for _, _, n in chunk)
             lens = [n for _, _, n in chunk]
             toks = np.concatenate([_int32(portions[i] if n == len(portions[i]) else portions[i][s:s + n]) for i, s, n in chunk])
+            slots = np.repeat(np.array([adapter_slots[i] for i, _, _ in chunk], dtype=np.int32), lens)  # (refuses more than 32 bits)
             passes, a = [], 0
             for i, _, n in chunk:
                 passes.append((seq_ids[i], a, n, kv.length(seq_ids[i])))
@@ -139,7 +140,7 @@ class EngineBase:
                             row_of[r] = len(rows)
                             rows.append(r)
                         dest.append((first_out[i] + k, row_of[r]))
-            self._stage_all((self.tokens, toks), (self.slots, np.repeat([adapter_slots[i] for i, _, _ in chunk], lens)),
+            self._stage_all((self.tokens, toks), (self.slots, slots),
                             (self.row_slot, row_slot), (self.row_pos, row_pos), (self.last_rows, rows or [T - 1]))
             self._begin_prompt_pass(passes)
             lg, tk = self.forward(T, False, use_lora, self.last_rows, max(len(rows), 1))

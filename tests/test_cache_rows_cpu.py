@@ -1,5 +1,6 @@
 """Rows of a forward as the host builds them: row by row against a plain list, over everything a caller may pass."""
 import random
+from types import SimpleNamespace
 
 import numpy as np
 import pytest
@@ -52,3 +53,17 @@ def test_unknown_sequences_and_too_many_pages_are_refused():
         kv.begin_rows([0, 9], [1, 1])
     with pytest.raises(RuntimeError):
         kv.begin_rows([0], [400])
+
+
+@pytest.mark.parametrize("slot", [1 << 32, 1 << 40, -(1 << 31) - 1])
+def test_adapter_slots_beyond_32_bits_are_refused(slot):
+    """... before anything is reserved, and not taken for what is left of them in 32 bits."""
+    base = load("engine").EngineBase
+    eng = base.__new__(base)
+    eng.kv, eng.m, eng.max_rows = _cache(), SimpleNamespace(device="cpu", V=8), 64
+    eng.tokens = eng.slots = eng.row_slot = eng.row_pos = eng.last_rows = None
+    eng.kv.add_sequence(4)
+    eng._stage_all = lambda *parts: pytest.fail("taken")
+    with pytest.raises(OverflowError):
+        eng.extend([4], [[1, 2, 3]], [slot])
+    assert eng.kv.tokens_reserved(4) == 0
