@@ -40,6 +40,21 @@ def test_base(T, K, N, packed, form):
     assert _err(y, ref) < (1e-5 if form == "f32" else TOL)
 
 
+# element by element: rounding to bf16 (2^-8 of the value), fp32 sums of K products (K 2^-24 of the sum of their magnitudes), and
+# what either activation makes of them (its slope is at most 1.13; a gelu of erff is good to 2^-20 of its argument)
+@pytest.mark.parametrize("T,K,N", [(9473, 200, 136), (160, 320, 12288), (257, 8, 12288 + 64), (1100, 320, 1920), (1999, 512, 2688)])
+@pytest.mark.parametrize("form", ["bf16", "gelu"])
+def test_every_element(T, K, N, form):
+    ops = load("ops")
+    _, x, W, _ = _setup(T, K, N, T + K)
+    z, slack = x.double() @ W.double().t(), (x.double().abs() @ W.double().abs().t()) * (K * 2.0 ** -24)
+    if form == "gelu":
+        slack = 1.13 * slack + 2.0 ** -20 * z.abs()
+        z = torch.nn.functional.gelu(z)
+    y = ops.linear(x, ops.PackedWeight(W), flags=ops.ACT_GELU if form == "gelu" else 0)
+    assert ((y.double() - z).abs() <= 2.0 ** -8 * z.abs() + (1 + 2.0 ** -8) * slack).all()
+
+
 # modules with odd numbers of row tiles (a pair must not span two of them); few adapters in runs, runs that start inside a
 # 16-row block, more than a run table holds, every row another adapter, none at all
 @pytest.mark.parametrize("rank", [16, 32, 64, 128])
