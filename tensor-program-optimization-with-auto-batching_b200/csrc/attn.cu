@@ -453,7 +453,7 @@ __global__ void __launch_bounds__(256) kv_append_rope_kernel(bf16* __restrict__ 
   }
 }
 
-// The same values in 16-byte pieces, where the key pages are aligned to that: a thread takes 8 dimensions of the first half of a
+// The same rotation (in fp32; a last bit may differ) in 16-byte pieces, where the key pages are aligned to that: a thread takes 8 dimensions of the first half of a
 // head and the 8 that rotate with them, and requests its pieces of two heads and of two value heads before it waits for the
 // row's sines and cosines (computed once per row, not once per thread) and its page.  Bound by HBM: a row is read and
 // written once.  Measured, 8192 rows, 32 + 2 x 32 heads of 128: 108 -> 80 us (403 MB, 5.0 TB/s); 1000 rows of 40 heads 17.9 -> 14.6.
@@ -558,7 +558,9 @@ extern "C" int mlora_kv_append_rope(void* d_qkv, int64_t ld, void* d_k_pages, vo
                 "kv_append_rope: null pointer");
   MLORA_REQUIRE(ld % 8 == 0 && aligned16(d_qkv) && aligned16(d_v_pages), "kv_append_rope: alignment");
   if (T == 0) return MLORA_OK;
-  const bool wide = aligned16(d_k_pages);  // (qkv and the value pages are: checked above)
+  // (qkv and the value pages are: checked above.  Key pages off a 16-byte border have always been taken here; this library's
+  // attention refuses them, a caller's own may not.)
+  const bool wide = aligned16(d_k_pages);
   launch_pdl(wide ? kv_append_rope16_kernel : kv_append_rope_kernel, T, kRope16Threads, 0, (cudaStream_t)stream, (bf16*)d_qkv, ld,
              (bf16*)d_k_pages, (bf16*)d_v_pages, d_block_table, max_pages, d_row_slot, d_row_pos, Hq, Hkv, D, page_size, rope_theta);
   count_launch();
