@@ -12,7 +12,7 @@
 //   O = O * exp2(m_old - m_new) + P V    in registers (128 fp32 per thread), while the tensor pipe is at the next S.
 // Scores are taken relative to the exact running maximum, so that the largest probability of a row is 1, which bf16 holds
 // exactly.  (A reference that lags behind the maximum, with O summed up in TMEM, is 5 % faster -- 354 us against 374 for 2 x 4096
-// rows -- but rounds dominating probabilities, which the sum does not see: 2 to 3.5 x the error for peaked rows.)
+// rows -- but rounds dominating probabilities, which the sum does not see: 1.7 to 3.4 x the error for peaked rows.)
 //
 // What bounds it: the softmax -- 16384 exponentials per block are 1024 cycles of an SM, the two MMAs are 1024 cycles of
 // tensor pipe -- and the chain S -> softmax -> P V of a CTA.  Two CTAs share an SM (96 KB of shared memory, 256 TMEM
