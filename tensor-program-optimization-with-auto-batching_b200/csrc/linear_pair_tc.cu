@@ -304,6 +304,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(LORA), 
           mbar_arrive(info_empty);
         }
       }
+      // the even CTA's last commits arrive in both CTAs: none of those arrivals may be on its way when a CTA leaves
+      for (int i = 0; i < NS && lane == 0 && ok && !s_abort; ++i, next()) {
+        if (!mbar_wait_pair(&empty_bar[s], par, &s_abort)) {
+          s_abort = 1;
+          atomicOr(p.status, 1);
+        }
+      }
     }
   } else if (warp == 1) {
     // ---- MMA issuer: one thread of the even CTA ----------------------------------------------------
@@ -609,6 +616,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(LORA), 
         ++n_batch;
       }
     }
+    if (ok) wait(cache_empty, (n_batch - 1) & 1);  // (as for the ring: the last batch's commit arrives in both CTAs)
   }
 
   // ---- teardown: the peer's copies, MMAs and arrivals reach into this CTA until the pair has met -------

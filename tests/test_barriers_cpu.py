@@ -45,3 +45,16 @@ def test_operand_builders_of_a_pair_share_a_verdict():
     role = src[src.index("const uint32_t cache_lead"):src.index("__syncthreads();\n  if (s_abort)")]
     assert role.count("mbar_wait_pair(") == 1  # in `wait` alone, which returns the role's verdict
     assert "return bar_all(2, w != 0);" in role
+
+
+def test_a_cta_of_a_pair_leaves_after_its_last_arrivals():
+    """Commits of the even CTA arrive at the odd one's barriers too: whoever uses a barrier waits for its last phase before the pair
+    parts (accumulators: the output warps wait for every one)."""
+    src = _source("linear_pair_tc.cu")
+    assert sorted(set(re.findall(r"umma_commit_pair\((?!uint32_t)(?:smem_u32\(&?)?(\w+)", src))) == ["acc_full", "cache_empty", "empty0"]
+    producer = src[src.index("const uint32_t full0 = lead_addr"):src.index("else if (warp == 1)")]
+    tail = producer[producer.index("mbar_arrive(info_empty)"):]
+    assert "i < NS" in tail and "mbar_wait_pair(&empty_bar[s], par" in tail
+    builders = src[src.index("const uint32_t cache_lead"):src.index("__syncthreads();\n  if (s_abort)")]
+    assert builders.index("++n_batch;") < builders.rindex("wait(cache_empty, (n_batch - 1) & 1);")
+    assert builders.rindex("wait(cache_empty") > builders.rindex("mbar_arrive_cluster(cache_lead)")
