@@ -80,6 +80,7 @@ def test_every_tile_is_dealt_exactly_once(T, K, N):
     assert n_tiles / slots > 0.6, "more than 40 % of the slots idle"
 
 
+# (of the one-CTA plan: prompt sizes run on it only where the expand is on CUDA cores, the others on pairs, below)
 def test_prompt_passes_take_256_token_tiles_and_decode_sizes_do_not():
     assert _plan(8192, 4096, 12288)["bn"] == 256
     assert _plan(8192, 4096, 4096)["bn"] == 256
