@@ -61,6 +61,10 @@ extern "C" {
                                CTAs only where that plan has whole tiles, whose sums are the same.  For projections in
                                front of a discrete choice (an expert router picks the largest of its scores): there
                                another order of fp32 sums is another choice at a near tie */
+#define MLORA_ANY_SUMS 2048 /* the caller does not need the sums over `in` in the order of mlora_linear_plan: up to 32 rows of
+                               a packed weight may run on the kernel that gives every CTA whole output rows.  Without this
+                               flag, or with MLORA_STABLE_SUMS, a call keeps the plan's sums, whose bits
+                               mlora_decode_chain reproduces */
 
 int mlora_version(void);
 const char* mlora_last_error(void);

@@ -340,6 +340,7 @@ int launch_linear_tc(const LinearArgs& a, void* work, size_t work_bytes, cudaStr
   const size_t need = linear_tc_workspace(a.T, a.in, a.out);
   if (work_bytes < need) return fail(MLORA_ESIZE, "linear: workspace of %zu bytes needed, %zu given", need, work_bytes);
   if (linear_pair_chosen(a)) return launch_linear_pair(a, work, st);
+  if (a.nf.res == nullptr && a.nf.sumsq_in == nullptr && linear_rows_chosen(a)) return launch_linear_rows(a, work, st);
   Plan pl = make_plan(a.T, a.in, a.out);
   switch (pl.bn) {
     case 16: return launch<16>(a, pl, work, st);

@@ -245,7 +245,7 @@ class PlainEngine(EngineBase):
     def _linear(self, x, W, out, flags=0):
         if self.m.dtype == torch.float32:  # (OUT_F32: what it writes anyway)
             return ops.linear_f32(x, W, flags & ~ops.OUT_F32, out=out)
-        return ops.linear(x, W, flags=flags, out=out, work=self.ws_linear)
+        return ops.linear(x, W, flags=flags | ops.ANY_SUMS, out=out, work=self.ws_linear)
 
 
 class DecodeGraph:

@@ -147,7 +147,7 @@ class MultiLoraLinear(nn.Module):
         slots = None
         if slots_per_batch_row is not None and stack is not None:
             slots = self._slot_tensor(slots_per_batch_row, x2.shape[0] // len(slots_per_batch_row), x2.device)
-        y = ops.linear(x2, Wp, stack if slots is not None else None, slots, with_shrink=True)
+        y = ops.linear(x2, Wp, stack if slots is not None else None, slots, flags=ops.ANY_SUMS, with_shrink=True)
         if self.base_layer.bias is not None:
             y = y + self.base_layer.bias.to(y.dtype)
         y = y.reshape(*lead, self.out_features)

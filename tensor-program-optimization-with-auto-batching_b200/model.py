@@ -29,7 +29,7 @@ import torch
 from . import ops
 from .engine import DecodeGraph, DecodeSession, EngineBase  # noqa: F401  (also reached as model.DecodeSession)
 from .kv_cache import PagedKVCache
-from .ops import LoraStack, LORA_PER_ROW, OUT_F32, SHARE_LORA_KERNEL, SILU_MUL
+from .ops import ANY_SUMS, LoraStack, LORA_PER_ROW, OUT_F32, SHARE_LORA_KERNEL, SILU_MUL
 
 ATTN_PROJ = ("q_proj", "k_proj", "v_proj", "o_proj")
 MLP_PROJ = ("gate_proj", "up_proj", "down_proj")
@@ -388,10 +388,10 @@ class Engine(EngineBase):
             r_tot = stack.r_max * stack.n_mod
             u = self.u.view(-1)[: T * r_tot].view(T, r_tot)
             ops.lora_shrink(x, stack, slots, out=u)
-            return ops.linear(x, W, stack, slots, u=u, flags=self._lora_flags(T, stack, flags), out=out,
+            return ops.linear(x, W, stack, slots, u=u, flags=ANY_SUMS | self._lora_flags(T, stack, flags), out=out,
                               work=self.ws_linear)
         # a projection without adapters inside a pass that has some: same kernel variant as its neighbours
-        return ops.linear(x, W, flags=flags | (SHARE_LORA_KERNEL if slots is not None else 0), out=out,
+        return ops.linear(x, W, flags=flags | ANY_SUMS | (SHARE_LORA_KERNEL if slots is not None else 0), out=out,
                           work=self.ws_linear)
 
     # ------------------------------------------------------------------------------------------
@@ -498,7 +498,7 @@ class Engine(EngineBase):
                 u = self.u.view(-1)[: T * r_tot].view(T, r_tot)
                 ops.residual_rmsnorm_shrink(delta, res, res_other, lw.ln1, m.eps, xn, st, slots, u)
                 res, res_other = res_other, res
-                ops.linear(xn, lw.w_qkv, st, slots, u=u, flags=self._lora_flags(T, st, 0), out=qkv, work=self.ws_linear)
+                ops.linear(xn, lw.w_qkv, st, slots, u=u, flags=ANY_SUMS | self._lora_flags(T, st, 0), out=qkv, work=self.ws_linear)
             else:
                 self._reduce_norm(delta, res, lw.ln1, xn, reduce=l > 0)
                 self._proj(xn, lw.w_qkv, st, slots, qkv)
@@ -535,9 +535,9 @@ class Engine(EngineBase):
                 self._proj(act, lw.w_down, lw.lora.get("down"), slots, y)
             else:
                 if lora_o:
-                    ops.linear(attn, lw.w_o, st_o, slots, u=u_o, flags=fl_o, out=y, work=self.ws_linear)
+                    ops.linear(attn, lw.w_o, st_o, slots, u=u_o, flags=fl_o | ANY_SUMS, out=y, work=self.ws_linear)
                 else:
-                    ops.linear(attn, lw.w_o, flags=fl_o, out=y, work=self.ws_linear)
+                    ops.linear(attn, lw.w_o, flags=fl_o | ANY_SUMS, out=y, work=self.ws_linear)
                 # row-parallel partials (base + LoRA) -> full o_proj output, added to the residual, normalised
                 self._reduce_norm(y, res, lw.ln2, xn)
                 if not self._mlp_chained(T, lw, slots, xn, act, y):
@@ -549,7 +549,7 @@ class Engine(EngineBase):
             xl = ops.embed(lm_rows[:n_lm], xn, out_bf16=self.xn_last[:n_lm])  # row gather
         else:
             n_lm, xl = T, xn
-        ops.linear(xl, m.lm_head, flags=OUT_F32 | (SHARE_LORA_KERNEL if slots is not None else 0), out=self.logits[:n_lm],
+        ops.linear(xl, m.lm_head, flags=OUT_F32 | ANY_SUMS | (SHARE_LORA_KERNEL if slots is not None else 0), out=self.logits[:n_lm],
                    work=self.ws_linear)
         ops.argmax(self.logits[:n_lm], out=self.next_tok[:n_lm])
         if m.tp_size > 1:

@@ -15,6 +15,7 @@ from ._lib import check
 
 OUT_F32, SILU_MUL, FORCE_SIMT, W_PACKED, B_PACKED, SHARE_LORA_KERNEL, LORA_PER_ROW, B_SPLIT = 1, 2, 4, 8, 16, 32, 64, 128
 STABLE_SUMS = 1024
+ANY_SUMS = 2048
 
 
 def _ptr(t):  # (plain numbers: the prototypes convert them)

@@ -335,6 +335,6 @@ class TevudraEngine(PlainEngine):
         rows = None if lm_rows is None else lm_rows[:n_lm]
         n = T if rows is None else n_lm
         self._norm(m.norm, T, add, rows)
-        self._linear(self.xn[:n], m.head, self.logits[:n], OUT_F32)
+        super()._linear(self.xn[:n], m.head, self.logits[:n], OUT_F32)  # (no router behind it)
         ops.argmax(self.logits[:n], out=self.next_tok[:n])
         return self.logits[:n], self.next_tok[:n]

@@ -1,0 +1,113 @@
+"""The decode-size projection that gives every CTA whole output rows (``MLORA_ANY_SUMS``): against float64 and the stream-K kernel."""
+import pytest
+import torch
+
+from conftest import load
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    return load("ops")
+
+
+def _run(ops, cuda, T, K, N, flags=0, rank=0, n_mod=1, n_ad=5, seed=0, ids=None):
+    """(output of this kernel, of stream-K, float64 reference, bound of one output's error)."""
+    g = torch.Generator().manual_seed(seed + T * 131 + K + N)
+    x = torch.randn(T, K, generator=g).bfloat16()
+    W = (torch.randn(N, K, generator=g) * K ** -0.5).bfloat16()
+    want = x.double() @ W.double().T
+    st = slots = u = None
+    if rank:
+        silu = flags & ops.SILU_MUL
+        pitch = 2 * rank if silu else rank  # (interleaved gate / up rows: one operand over both modules' ranks)
+        B = (torch.randn(n_ad, N, pitch, generator=g) * 0.1).bfloat16()
+        u = torch.randn(T, rank * n_mod, generator=g)
+        slots = torch.randint(-1, n_ad + 1, (T,), generator=g).int() if ids is None else torch.tensor(ids).int()  # n_ad: no such adapter
+        offs = (0, N) if silu or n_mod == 1 else tuple(N // 128 * i // n_mod * 128 for i in range(n_mod)) + (N,)
+        scales = torch.linspace(0.5, 2.0, n_ad)
+        for t in range(T):
+            s = int(slots[t])
+            if not 0 <= s < n_ad:
+                continue
+            su = (scales[s] * u[t]).bfloat16().double()  # (the operand both kernels multiply)
+            for m in range(1 if silu else n_mod):
+                lo, hi = (0, N) if silu else (offs[m], offs[m + 1])
+                want[t, lo:hi] += B[s, lo:hi].double() @ (su if silu else su[m * rank:(m + 1) * rank])
+        st = ops.LoraStack(torch.zeros(n_ad, rank * n_mod, K, dtype=torch.bfloat16, device=cuda), B.to(cuda),
+                           torch.full((n_ad,), rank, dtype=torch.int32, device=cuda), scales.to(cuda), rank, n_mod, offs).pack_b()
+        u, slots = u.to(cuda), slots.to(cuda)
+    if flags & ops.SILU_MUL:
+        v = want.view(T, -1, 2, 8)
+        want = (v[:, :, 0] * torch.sigmoid(v[:, :, 0]) * v[:, :, 1]).reshape(T, -1)
+    elif flags & ops.ACT_RELU2:
+        want = want.clamp(min=0) ** 2
+    elif flags & ops.ACT_GELU:
+        want = 0.5 * want * (1 + torch.erf(want / 2 ** 0.5))
+    work = ops.new_workspace(load("_lib").lib().mlora_linear_workspace(T, K, N), cuda)
+    got, old = (ops.linear(x.to(cuda), ops.PackedWeight(W.to(cuda)), st, slots, u=u, flags=flags | f, work=work) for f in (ops.ANY_SUMS, 0))
+    again = ops.linear(x.to(cuda), ops.PackedWeight(W.to(cuda)), st, slots, u=u, flags=flags | ops.ANY_SUMS, work=work)
+    assert ops.status_word(work) == 0
+    assert torch.equal(got, again)  # a fixed order of sums
+    return got.double().cpu(), old.double().cpu(), want
+
+
+def _check(got, old, want, f32):
+    # fp32 sums of some thousand products: below 2^-16 of the result's size; bf16 outputs: half a unit in the last of 8 bits, 2^-8 of a
+    # value.  No further off than stream-K, but for sums so short that both are at fp32's own rounding (2^-20 of the result)
+    size = want.abs().max()
+    err, err_old = (got - want).abs(), (old - want).abs()
+    assert float((err - (0 if f32 else 2 ** -8) * want.abs()).max()) <= 2 ** -16 * float(size)
+    assert float(err.norm()) <= (1.0 if f32 else 1.01) * float(err_old.norm()) + 2 ** -20 * float(want.norm())
+
+
+@pytest.mark.parametrize("T", [1, 15, 16, 17, 32])
+@pytest.mark.parametrize("K,N", [(8, 1184), (72, 1200), (512, 2048), (1032, 4096), (4096, 7000), (4096, 9600), (4096, 12288), (3072, 20104), (4096, 28424),
+                                 (8192, 2048), (16384, 4096)])
+def test_plain(ops, cuda, T, K, N):
+    """One row group per CTA and several, one to three passes, odd numbers of k-blocks, ragged last rows, slots of 2 to 8 k-blocks."""
+    _check(*_run(ops, cuda, T, K, N, ops.OUT_F32), True)
+
+
+@pytest.mark.parametrize("T", [3, 32])
+@pytest.mark.parametrize("flag", ["SILU_MUL", "ACT_RELU2", "ACT_GELU", None])
+@pytest.mark.parametrize("K,N", [(256, 1200), (640, 2064), (2048, 22016)])
+def test_activations_and_bf16(ops, cuda, T, flag, K, N):
+    _check(*_run(ops, cuda, T, K, N, getattr(ops, flag) if flag else 0), False)
+
+
+@pytest.mark.parametrize("T,rank,n_mod,K,N", [(1, 16, 1, 4096, 4096), (16, 16, 3, 1024, 12288), (17, 32, 3, 512, 1536), (32, 64, 3, 4096, 12288),
+                                              (32, 128, 1, 256, 1208), (9, 64, 1, 11008, 4096), (32, 16, 8, 128, 2048)])
+def test_adapters(ops, cuda, T, rank, n_mod, K, N):
+    """Module boundaries inside a CTA's rows, adapters over several slots, rows without adapter or with one that does not exist."""
+    _check(*_run(ops, cuda, T, K, N, ops.OUT_F32, rank, n_mod), True)
+
+
+def test_adapters_all_distinct_none_and_gate_up(ops, cuda):
+    _check(*_run(ops, cuda, 32, 512, 4096, ops.OUT_F32, 16, 1, 32, ids=list(range(32))), True)
+    _check(*_run(ops, cuda, 32, 512, 4096, ops.OUT_F32, 16, 1, 4, ids=[-1] * 32), True)
+    for T in (5, 32):
+        _check(*_run(ops, cuda, T, 512, 22016, ops.SILU_MUL, 64, 2), False)
+
+
+def test_rows_and_outputs_of_other_pitches(ops, cuda):
+    """x as a slice of wider rows; y likewise, also where four outputs are no aligned store."""
+    g = torch.Generator().manual_seed(1)
+    X, W = torch.randn(7, 520, generator=g).bfloat16().to(cuda), (torch.randn(1192, 256, generator=g) / 16).bfloat16().to(cuda)
+    x, Y = X[:, 8:264], torch.full((7, 1229), 9.0, dtype=torch.bfloat16, device=cuda)
+    work = ops.new_workspace(load("_lib").lib().mlora_linear_workspace(7, 256, 1192), cuda)
+    ops.linear(x, ops.PackedWeight(W), flags=ops.ANY_SUMS, out=Y[:, 3:1195], work=work)
+    want = x.double() @ W.double().T
+    assert float(((Y[:, 3:1195].double() - want).abs() - 2 ** -8 * want.abs()).max()) < 1e-4
+    assert bool((Y[:, :3] == 9).all()) and bool((Y[:, 1195:] == 9).all())
+
+
+def test_calls_that_keep_the_plans_sums(ops, cuda):
+    """Without the flag, or with STABLE_SUMS, the bits are those of the stream-K plan."""
+    got = {}
+    g = torch.Generator().manual_seed(2)
+    x, W = torch.randn(4, 4096, generator=g).bfloat16().to(cuda), ops.PackedWeight(torch.randn(4096, 4096, generator=g).bfloat16().to(cuda))
+    for f in (0, ops.STABLE_SUMS, ops.STABLE_SUMS | ops.ANY_SUMS):
+        got[f] = ops.linear(x, W, flags=f | ops.OUT_F32)
+    assert torch.equal(got[0], got[ops.STABLE_SUMS]) and torch.equal(got[0], got[ops.STABLE_SUMS | ops.ANY_SUMS])
