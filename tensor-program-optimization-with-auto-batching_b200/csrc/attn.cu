@@ -361,6 +361,321 @@ __global__ void __launch_bounds__(128) paged_attn_kernel(AttnArgs a) {
   }
 }
 
+// The same with REP query heads that share a key head in one CTA: its keys and values are read once instead of once per query
+// head.  (L2 gave them back, but that path was the limit: 32 heads over 8 key heads, 32 rows of 512 to 1024 keys 45.8 -> 32.0 us with
+// 15.5 us of bytes, of 8192 keys 410 -> 198 with 166.)  A page's REP x 8 scores of a lane group are summed over its 16 lanes by
+// halving exchanges -- every step keeps half of the values -- so that each lane ends with REP / 2 of them and the exponentials are
+// taken once, not sixteen times.  The next page's keys are requested as soon as a page's scores are known, its values as soon
+// as they are summed up.  Two CTAs per SM at four heads: held to three (168 registers, spills) the same rows take 40.9 and 268 us; at two
+// heads four CTAs (32 over 16 heads, 512 keys 24.6 us, 32.8 with two).  Heads of 128 columns, pages of 16 and 32; grid (Hq / REP, T, n_splits).
+typedef unsigned long long f32x2;  // two fp32 values in one register pair
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+// 8 bf16 -> four pairs
+__device__ __forceinline__ void unpack8x2(const uint4& v, f32x2 (&f)[4]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[i] = pack2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xffff0000u));
+}
+
+template <int PS, int REP, bool RMS>
+__global__ void __launch_bounds__(128, REP == 4 ? 2 : 4) paged_attn_group_kernel(AttnArgs a) {
+  constexpr int D = 128, IT = 8, R = REP / 2, LPH = IT / R;  // LPH: lanes that hold the scores of a head
+  static_assert(REP == 2 || REP == 4, "scores per lane");
+  __shared__ float sq[REP][D];
+  __shared__ float sk[D], sv[D];
+  __shared__ float wm[4][REP], wl[4][REP];
+  __shared__ float wacc[4][REP][D];
+  __shared__ float s_new[REP];
+
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.y, split = blockIdx.z, h0 = blockIdx.x * REP;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int rep = a.Hq / a.Hkv, kvh = h0 / rep;
+  const int slot = a.row_slot[t], pos = a.row_pos[t];
+  const int32_t* bt = a.block_table + (size_t)slot * a.max_pages;
+  const bf16* row = a.qkv + (size_t)t * a.ld;
+  const bool last_split = split == a.n_splits - 1;
+  const bool has_new = a.fused && last_split;
+  const bool can_store = pos >= 0 && pos / PS < a.max_pages;  // (as above)
+  const bool stores = has_new && h0 % rep == 0 && can_store;
+
+  const int n_tok = min(max(a.fused ? pos : pos + 1, 0), a.max_pages * PS);
+  const int n_pg = (n_tok + PS - 1) / PS;
+  const int lo = (a.chunk > 0 && pos > 0) ? pos - pos % a.chunk : 0;
+  const int pg_lo = min(lo / PS, n_pg);
+  const int per = (n_pg - pg_lo + a.n_splits - 1) / a.n_splits;
+  const int pg_begin = min(pg_lo + split * per, n_pg), pg_end = min(pg_begin + per, n_pg);
+  const int g = lane >> 4, dl = lane & 15, base = lane & 16;
+  const uint64_t pol = kv_policy();
+  constexpr int SUB = PS / 16;  // steps of 16 tokens
+  const int st_end = pg_end * SUB;
+  uint4 kr[IT], vr[IT];
+  auto place = [&](int st) { return ((size_t)bt[st / SUB] * a.Hkv + kvh) * PS * D + (size_t)((st % SUB) * 16 + g) * D + dl * 8; };
+  auto load = [&](uint4 (&r)[IT], const bf16* pages, size_t at) {
+#pragma unroll
+    for (int it = 0; it < IT; ++it) r[it] = ld_kv(pages + at + it * 2 * D, pol);
+  };
+  int st = pg_begin * SUB + warp;
+  if (st < st_end) {  // the first page is on its way during the prologue
+    const size_t at = place(st);
+    load(kr, a.k_pages, at);
+    load(vr, a.v_pages, at);
+  }
+
+  // ---- prologue: thread = column; rotate the queries (and the new key), stage the new key and value ----
+  {
+    const int d = tid;
+    if constexpr (RMS) {
+      __shared__ float s_sum[REP + 1][4];
+      const int half = a.rot / 2, o = d < half ? d + half : d - half;  // the column it is paired with, if it is rotated
+      const auto value = [&](int head, int c) {
+        return __bfloat162float(row[(size_t)head * a.dim + c]) + (a.bias ? a.bias[(size_t)head * a.dim + c] : 0.f);
+      };
+      float y[REP + 1], kx = 0.f, sn = 0.f, cs = 1.f;
+      const bool turned = d < a.rot && d < a.dim;
+      if (turned) {
+        sincosf((float)pos * a.inv_freq[d < half ? d : o], &sn, &cs);
+        if (d < half) sn = -sn;
+      }
+      float z[REP + 1];  // the paired columns; everything is requested before anything is used
+#pragma unroll
+      for (int i = 0; i <= REP; ++i) {
+        const int head = i < REP ? h0 + i : a.Hq + kvh;
+        y[i] = d < a.dim ? value(head, d) : 0.f;
+        z[i] = turned ? value(head, o) : 0.f;
+      }
+      kx = y[REP];
+#pragma unroll
+      for (int i = 0; i <= REP; ++i) {
+        if (turned) y[i] = fmaf(y[i], cs, z[i] * sn);
+        const float ss = warp_sum(y[i] * y[i]);
+        if (lane == 0) s_sum[i][warp] = ss;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i <= REP; ++i) {
+        const float n = (s_sum[i][0] + s_sum[i][1]) + (s_sum[i][2] + s_sum[i][3]);
+        y[i] *= 1.f / sqrtf(n / (float)a.dim + a.eps);
+        if (i < REP) sq[i][d] = y[i] * a.qscale;
+      }
+      const bf16 kr = __float2bfloat16_rn(y[REP]), vr = __float2bfloat16_rn(kx);
+      sk[d] = __bfloat162float(kr);
+      sv[d] = __bfloat162float(vr);
+      if (stores) {
+        const size_t at = (((size_t)bt[pos / PS] * a.Hkv + kvh) * PS + pos % PS) * D + d;
+        a.k_pages[at] = kr;
+        a.v_pages[at] = vr;
+      }
+    } else {
+      const int i = d & (D / 2 - 1);  // the pair (i, i + D / 2); the lower half of the threads turns it for the upper half too
+      if (d < D / 2) {
+        float sn = 0.f, cs = 1.f;
+        if (a.fused) sincosf((float)pos * rope_inv_freq(a.theta, i, D), &sn, &cs);
+#pragma unroll
+        for (int j = 0; j < REP; ++j) {
+          const float q1 = __bfloat162float(row[(h0 + j) * D + i]), q2 = __bfloat162float(row[(h0 + j) * D + i + D / 2]);
+          sq[j][i] = (a.fused ? q1 * cs - q2 * sn : q1) * a.qscale;
+          sq[j][i + D / 2] = (a.fused ? q2 * cs + q1 * sn : q2) * a.qscale;
+        }
+        if (has_new) {
+          const bf16* kr = row + (size_t)(a.Hq + kvh) * D;
+          const float k1 = __bfloat162float(kr[i]), k2 = __bfloat162float(kr[i + D / 2]);
+          const bf16 r1 = __float2bfloat16_rn(k1 * cs - k2 * sn), r2 = __float2bfloat16_rn(k2 * cs + k1 * sn);
+          sk[i] = __bfloat162float(r1);
+          sk[i + D / 2] = __bfloat162float(r2);
+          if (stores) {
+            bf16* dst = a.k_pages + (((size_t)bt[pos / PS] * a.Hkv + kvh) * PS + pos % PS) * D;
+            dst[i] = r1;
+            dst[i + D / 2] = r2;
+          }
+        }
+      }
+      if (has_new) {
+        const bf16 v = row[(size_t)(a.Hq + a.Hkv + kvh) * D + d];
+        sv[d] = __bfloat162float(v);
+        if (stores) a.v_pages[(((size_t)bt[pos / PS] * a.Hkv + kvh) * PS + pos % PS) * D + d] = v;
+      }
+    }
+  }
+  __syncthreads();
+
+  f32x2 qf[REP][4];
+#pragma unroll
+  for (int j = 0; j < REP; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) qf[j][e] = pack2(sq[j][dl * 8 + 2 * e], sq[j][dl * 8 + 2 * e + 1]);
+
+  // m, l: of the head whose scores this lane holds (l only this lane's share); acc: eight columns of every head
+  float m = -INFINITY, l = 0.f;
+  f32x2 acc2[REP][4];
+#pragma unroll
+  for (int j = 0; j < REP; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc2[j][e] = 0ull;
+
+  while (st < st_end) {
+    const int key0 = st * 16, next = st + 4;
+    const size_t at = next < st_end ? place(next) : 0;
+    float v[REP * IT];
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      f32x2 kf[4];
+      unpack8x2(kr[it], kf);
+#pragma unroll
+      for (int j = 0; j < REP; ++j) {
+        f32x2 d = fma2(qf[j][0], kf[0], 0ull);
+#pragma unroll
+        for (int e = 1; e < 4; ++e) d = fma2(qf[j][e], kf[e], d);
+        const float2 h = unpack2(d);
+        v[j * IT + it] = h.x + h.y;
+      }
+    }
+    if (next < st_end) load(kr, a.k_pages, at);
+#pragma unroll
+    for (int o = 8, n = REP * IT / 2; o >= 1; o >>= 1, n >>= 1) {
+      const bool up = (dl & o) != 0;
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        const float send = up ? v[i] : v[i + n], keep = up ? v[i + n] : v[i];
+        v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    }
+    // v[r] = the score of head (dl R + r) / 8 and token 2 ((dl R + r) mod 8) + g of the step
+    float p[R], mx = -INFINITY;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int key = key0 + ((dl * R + r) & 7) * 2 + g;
+      p[r] = key < n_tok && key >= lo ? v[r] : -INFINITY;
+      mx = fmaxf(mx, p[r]);
+    }
+#pragma unroll
+    for (int o = 1; o < LPH; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float mn = fmaxf(m, mx);
+    if (__any_sync(0xffffffffu, mn > m)) {
+      const float corr = m == -INFINITY ? 0.f : exp2f(m - mn);
+      l *= corr;
+#pragma unroll
+      for (int j = 0; j < REP; ++j) {
+        const float c = __shfl_sync(0xffffffffu, corr, base + j * LPH);
+        const f32x2 c2 = pack2(c, c);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc2[j][e] = fma2(acc2[j][e], c2, 0ull);
+      }
+      m = mn;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      p[r] = p[r] == -INFINITY ? 0.f : exp2f(p[r] - m);
+      l += p[r];
+    }
+    if (key0 + 16 > n_tok || key0 < lo) {  // a key that is not seen has probability 0, but its value may be anything
+#pragma unroll
+      for (int it = 0; it < IT; ++it)
+        if (key0 + it * 2 + g >= n_tok || key0 + it * 2 + g < lo) vr[it] = make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int it = 0; it < IT; ++it) {
+      f32x2 vf[4];
+      unpack8x2(vr[it], vf);
+#pragma unroll
+      for (int j = 0; j < REP; ++j) {
+        const float pj = __shfl_sync(0xffffffffu, p[it % R], base + j * LPH + it / R);
+        const f32x2 pp = pack2(pj, pj);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc2[j][e] = fma2(pp, vf[e], acc2[j][e]);
+      }
+    }
+    if (next < st_end) load(vr, a.v_pages, at);
+    st = next;
+  }
+  float acc[REP][8];
+#pragma unroll
+  for (int j = 0; j < REP; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 t2 = unpack2(acc2[j][e]);
+      acc[j][2 * e] = t2.x;
+      acc[j][2 * e + 1] = t2.y;
+    }
+
+  // ---- merge the two lane groups of the warp, then the warps (+ the new token), and write -----------------
+#pragma unroll
+  for (int o = 1; o < LPH; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+#pragma unroll
+  for (int j = 0; j < REP; ++j) {
+    float mj = __shfl_sync(0xffffffffu, m, base + j * LPH), lj = __shfl_sync(0xffffffffu, l, base + j * LPH);
+    const float mo = __shfl_xor_sync(0xffffffffu, mj, 16), lo2 = __shfl_xor_sync(0xffffffffu, lj, 16);
+    float ao[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) ao[e] = __shfl_xor_sync(0xffffffffu, acc[j][e], 16);
+    merge_state(mj, lj, acc[j], mo, lo2, ao);
+    if (lane < 16) {
+      if (lane == 0) {
+        wm[warp][j] = mj;
+        wl[warp][j] = lj;
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) wacc[warp][j][lane * 8 + e] = acc[j][e];
+    }
+  }
+  if (has_new && warp < REP) {
+    float d = 0.f;
+    for (int i = lane; i < D; i += 32) d = fmaf(sq[warp][i], sk[i], d);
+    d = warp_sum(d);
+    if (lane == 0) s_new[warp] = d;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < REP; ++j) {
+    const int h = h0 + j;
+    float M = has_new ? s_new[j] : -INFINITY;
+    const float sink = (a.sink && last_split) ? a.sink[h] * kLog2e : -INFINITY;
+    M = fmaxf(M, sink);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) M = fmaxf(M, wm[w][j]);
+    float L = 0.f, O = 0.f;
+    if (M != -INFINITY) {
+      if (sink != -INFINITY) L = exp2f(sink - M);
+#pragma unroll
+      for (int w = 0; w < 4; ++w) {
+        const float c = wm[w][j] == -INFINITY ? 0.f : exp2f(wm[w][j] - M);
+        L = fmaf(wl[w][j], c, L);
+        O = fmaf(wacc[w][j][tid], c, O);
+      }
+      if (has_new) {
+        const float c = exp2f(s_new[j] - M);
+        L += c;
+        O = fmaf(sv[tid], c, O);
+      }
+    }
+    if (a.n_splits == 1) {
+      a.out[(size_t)t * a.ld_out + h * D + tid] = __float2bfloat16_rn(L > 0.f ? O / L : 0.f);
+    } else {
+      float* w = a.work + (((size_t)t * a.Hq + h) * a.n_splits + split) * (D + 2);
+      w[tid] = O;
+      if (tid == 0) {
+        w[D] = M;
+        w[D + 1] = L;
+      }
+    }
+  }
+}
+
 // grid (Hq, T), D threads: combine the n_splits partial results of one (row, head).
 constexpr int kMergeAtOnce = 16;
 __global__ void attn_merge_kernel(const float* __restrict__ work, int Hq, int D, int n_splits,
@@ -620,7 +935,20 @@ static int attention_impl(const void* d_qkv, int64_t ld, void* d_k_pages, void* 
   dim3 grid(Hq, T, n_splits);
   cudaStream_t st = (cudaStream_t)stream;
   const auto go = [&](auto plain, auto rms) { launch_pdl_if(pdl_enabled_attn(), nt.dim ? rms : plain, grid, 128, 0, st, a); };
-  if (D == 128 && page_size == 16)
+  // Query heads that share a key head go together, four or two at a time (the shrink tail is laid out by single heads).  A warp
+  // takes longer over a page then, so with few rows single heads on more CTAs are faster: 4 rows of 16 heads over 4, 100 keys 5.5 us
+  // against 8.3, 1 row of 32 heads over 8, 2000 keys 11.3 / 12.7; 16 rows x 32 heads 28.9 / 22.6, 19 rows 37.4 / 26.3.
+  const int rep = Hq / Hkv, group = sh.A || D != 128 || (long long)T * Hq < 512 ? 1 : rep % 4 == 0 ? 4 : rep % 2 == 0 ? 2 : 1;
+  grid.x = Hq / group;
+  if (group == 4 && page_size == 16)
+    go(paged_attn_group_kernel<16, 4, false>, paged_attn_group_kernel<16, 4, true>);
+  else if (group == 4)
+    go(paged_attn_group_kernel<32, 4, false>, paged_attn_group_kernel<32, 4, true>);
+  else if (group == 2 && page_size == 16)
+    go(paged_attn_group_kernel<16, 2, false>, paged_attn_group_kernel<16, 2, true>);
+  else if (group == 2)
+    go(paged_attn_group_kernel<32, 2, false>, paged_attn_group_kernel<32, 2, true>);
+  else if (D == 128 && page_size == 16)
     go(paged_attn_kernel<128, 8, false>, paged_attn_kernel<128, 8, true>);
   else if (D == 128 && page_size == 32)
     go(paged_attn_kernel<128, 16, false>, paged_attn_kernel<128, 16, true>);

@@ -111,3 +111,13 @@ def test_calls_that_keep_the_plans_sums(ops, cuda):
     for f in (0, ops.STABLE_SUMS, ops.STABLE_SUMS | ops.ANY_SUMS):
         got[f] = ops.linear(x, W, flags=f | ops.OUT_F32)
     assert torch.equal(got[0], got[ops.STABLE_SUMS]) and torch.equal(got[0], got[ops.STABLE_SUMS | ops.ANY_SUMS])
+
+
+@pytest.mark.parametrize("T,rank,n_mod", [(16, 64, 3), (32, 16, 1), (20, 64, 1)])
+def test_many_distinct_adapters_take_the_ring(ops, cuda, T, rank, n_mod):
+    """``LORA_PER_ROW`` asks for the expand of distinct adapters: here the same launch as without it, y rounded once."""
+    ids = list(range(T))
+    got, _, want = _run(ops, cuda, T, 1024, 3072, ops.LORA_PER_ROW, rank, n_mod, T, ids=ids)
+    plain, _, _ = _run(ops, cuda, T, 1024, 3072, 0, rank, n_mod, T, ids=ids)
+    assert torch.equal(got, plain)
+    assert float(((got - want).abs() - 2 ** -8 * want.abs()).max()) <= 2 ** -16 * float(want.abs().max())
