@@ -386,6 +386,14 @@ int mlora_paged_attention_static(const void* d_qkv, int64_t ld, void* d_k_pages,
                                  float rope_theta, int32_t fused_append, void* d_out, int64_t ld_out,
                                  int32_t n_splits, void* stream);
 
+/* Host values to a device table through the launch's own parameters (896 values per launch): d_dst[i] = h_values[i / repeat],
+ * i < n * repeat.  h_values may be changed as soon as the call returns. */
+int mlora_put_i32(int32_t* d_dst, const int32_t* h_values, int32_t n, int32_t repeat, void* stream);
+
+/* The row tables of a prompt pass from one record per sequence, h_seqs [n][4] = cache slot, adapter slot, rows (>= 0), position of
+ * its first row; rows lie one sequence behind the other: d_slots / d_row_slot / d_row_pos [sum of rows]. */
+int mlora_put_rows(const int32_t* h_seqs, int32_t n, int32_t* d_slots, int32_t* d_row_slot, int32_t* d_row_pos, void* stream);
+
 /* ---- decode-step bookkeeping on the device (keeps a whole step inside one CUDA graph) ----------
  * For each live row b: slot = d_row_slot[b]; d_row_pos[b] = d_seq_lens[slot]; d_seq_lens[slot] += 1.
  * What kv_state_begin_forward(kv, seq_ids, [1]*B) does on the host in the reference

@@ -63,6 +63,8 @@ PROTOTYPES = {
     "mlora_paged_attention_static_max_bytes": (_sz, []),
     "mlora_paged_attention_static": (C.c_int, [_vp, _i64, _vp, _vp, _vp, _i32, _vp, _vp, _i32, _i32, _i32, _i32, _i32,
                                                _f32, _i32, _vp, _i64, _i32, _vp]),
+    "mlora_put_i32": (C.c_int, [_vp, _vp, _i32, _i32, _vp]),
+    "mlora_put_rows": (C.c_int, [_vp, _i32, _vp, _vp, _vp, _vp]),
     "mlora_kv_begin_decode": (C.c_int, [_vp, _vp, _vp, _i32, _vp]),
     "mlora_tp_arena_bytes": (_sz, [_i32, _i32]),
     "mlora_tp_create": (C.c_int, [_i32, _i32, _i32, _i32, C.POINTER(_vp)]),

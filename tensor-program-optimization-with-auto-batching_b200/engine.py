@@ -33,7 +33,7 @@ class EngineBase:
     adapter slots, ``row_slot`` = cache slots, ``row_pos``), returning (logits, next tokens);
     ``_begin_prompt_pass(chunk)`` / ``_end_prompt_pass()`` around the forward of a prompt pass, ``chunk`` a list of
     (sequence id, first row, rows, position of the first row);
-    ``_check_prompt_status()`` after the last pass of a call."""
+    kernels with bounded waits report to ``_own_status_word()``."""
 
     def __init__(self, model, kv: PagedCache, max_rows: int):
         self.m, self.kv, self.max_rows = model, kv, int(max_rows)
@@ -60,30 +60,43 @@ class EngineBase:
     def _end_prompt_pass(self):
         pass
 
-    def _check_prompt_status(self):
-        pass
-
     def status_word(self) -> int:
         """Status word of the projection kernels' scratch (synchronises): non-zero after a bounded wait expired
         somewhere since the buffer was last cleared; the outputs since then are undefined."""
         return ops.status_word(self.ws_linear)
 
+    def _own_status_word(self):
+        """A word of the projection scratch's header that no projection uses, for the engine's other kernels with bounded waits:
+        :meth:`check_status` reads both words at once."""
+        return self.ws_linear[240:244].view(torch.int32)
+
     def check_status(self):
-        """Raises if a projection kernel gave up a bounded wait, after re-zeroing the scratch (arrival counters of
-        split tiles may be stale after such a failure) so that the engine stays usable."""
-        st = self.status_word()
-        if st:
+        """Raises if a kernel gave up a bounded wait, after re-zeroing the scratch (arrival counters of split tiles may be stale
+        after such a failure) so that the engine stays usable."""
+        words = self.ws_linear[:244].view(torch.int32).tolist()
+        st, own = words[0], words[60]
+        if st or own:
             self.ws_linear.zero_()
+        if st:
             raise RuntimeError(f"mlora: a projection kernel gave up a bounded wait (status bits {st:#x}); "
                                "the results of this pass are undefined")
+        if own:
+            raise RuntimeError("mlora: an attention kernel gave up a bounded wait; this pass's results are undefined")
 
     def _stage(self, dst, values, dtype):
         t = torch.as_tensor(np.asarray(values), dtype=dtype)
         dst[: t.numel()].copy_(t.pin_memory(), non_blocking=True)
 
     def _stage_all(self, *parts):
-        """Copies int32 arrays to the starts of device buffers: (buffer, array) pairs, through one pinned buffer."""
+        """Copies int32 arrays to the starts of device buffers: (buffer, array) pairs; small ones in launch parameters, the others
+        through one pinned buffer."""
         parts = [(dst, np.asarray(v, dtype=np.int32).reshape(-1)) for dst, v in parts]
+        for dst, v in parts:
+            if v.size <= ops.PUT_AT_MOST:
+                ops.put_i32(dst, v)
+        parts = [(dst, v) for dst, v in parts if v.size > ops.PUT_AT_MOST]
+        if not parts:
+            return
         pinned = torch.from_numpy(np.concatenate([v for _, v in parts])).pin_memory()
         a = 0
         for dst, v in parts:
@@ -123,12 +136,13 @@ class EngineBase:
             T = sum(n for _, _, n in chunk)
             lens = [n for _, _, n in chunk]
             toks = np.concatenate([_int32(portions[i] if n == len(portions[i]) else portions[i][s:s + n]) for i, s, n in chunk])
-            slots = np.repeat(np.array([adapter_slots[i] for i, _, _ in chunk], dtype=np.int32), lens)  # (refuses more than 32 bits)
+            seqs = np.empty((len(chunk), 4), dtype=np.int32)
+            seqs[:, 1] = np.array([adapter_slots[i] for i, _, _ in chunk], dtype=np.int32)  # (refuses more than 32 bits)
             passes, a = [], 0
             for i, _, n in chunk:
                 passes.append((seq_ids[i], a, n, kv.length(seq_ids[i])))
                 a += n
-            row_slot, row_pos = kv.begin_rows([seq_ids[i] for i, _, _ in chunk], lens)
+            seqs[:, 0], seqs[:, 3], seqs[:, 2] = kv.begin_ranges([seq_ids[i] for i, _, _ in chunk], lens)
             self.n_distinct = len({int(adapter_slots[i]) for i, _, _ in chunk if adapter_slots[i] >= 0})
             self.max_keys = max(p0 + n for _, _, n, p0 in passes)
             rows, dest, row_of = [], [], {}
@@ -140,8 +154,8 @@ class EngineBase:
                             row_of[r] = len(rows)
                             rows.append(r)
                         dest.append((first_out[i] + k, row_of[r]))
-            self._stage_all((self.tokens, toks), (self.slots, slots),
-                            (self.row_slot, row_slot), (self.row_pos, row_pos), (self.last_rows, rows or [T - 1]))
+            ops.put_rows(seqs, self.slots, self.row_slot, self.row_pos)
+            self._stage_all((self.tokens, toks), (self.last_rows, rows or [T - 1]))
             self._begin_prompt_pass(passes)
             lg, tk = self.forward(T, False, use_lora, self.last_rows, max(len(rows), 1))
             if rows:
@@ -156,7 +170,6 @@ class EngineBase:
             kv.end_forward()
             self._end_prompt_pass()
         self.check_status()  # (synchronises; prefill is not the latency-critical call)
-        self._check_prompt_status()
         return out_logits, out_tok
 
     def prefill(self, seq_ids, prompts, adapter_slots, use_lora=True):
@@ -223,7 +236,7 @@ class PlainEngine(EngineBase):
         # (some projections have more rows than the pass: scratch no longer grows beyond 128)
         need = max([work_bytes] + [lib.mlora_linear_workspace(max(T, 128), k, n) for k, n in linears])
         self.ws_linear = ops.new_workspace(need, model.device)
-        self.status = torch.zeros(1, dtype=torch.int32, device=model.device)
+        self.status = self._own_status_word()
         self._buf, self._retired = {}, []
 
     # -- buffers that only some passes need, grown on demand (never while a graph is being captured: its warm-up run
@@ -235,12 +248,6 @@ class PlainEngine(EngineBase):
                 self._retired.append(t)
             t = self._buf[name] = torch.zeros(numel, dtype=dtype or self.m.dtype, device=self.m.device)
         return t[:numel]
-
-    def check_status(self):
-        super().check_status()
-        if int(self.status.item()):
-            self.status.zero_()
-            raise RuntimeError("mlora: an attention kernel gave up a bounded wait; this pass's results are undefined")
 
     def _linear(self, x, W, out, flags=0):
         if self.m.dtype == torch.float32:  # (OUT_F32: what it writes anyway)

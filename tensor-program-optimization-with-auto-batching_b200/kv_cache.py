@@ -56,10 +56,13 @@ class PagedCache:
         self._slot_of[sid] = slot
         self._n_pages_of[sid] = 0
         self._len_host[slot] = 0
-        self.seq_lens[slot:slot + 1].zero_()  # (a fill: no staging buffer)
+        self._push(self.seq_lens[slot:slot + 1], self._len_host[slot:slot + 1])
         return slot
 
     def _push(self, dst, src_np):
+        if dst.is_cuda and src_np.size <= ops.PUT_AT_MOST and dst.is_contiguous():
+            ops.put_i32(dst, src_np)
+            return
         dst.copy_(torch.from_numpy(np.ascontiguousarray(src_np)).pin_memory(), non_blocking=True)
 
     def remove_sequence(self, sid):
@@ -125,6 +128,14 @@ class PagedCache:
 
     def begin_rows(self, seq_ids, append_lens):
         """:meth:`begin_forward` for a caller that uploads the rows with others of its own: two int32 arrays on the host."""
+        slots, first, lens = self.begin_ranges(seq_ids, append_lens)
+        lens = np.maximum(lens, 0)  # a negative length takes tokens back at the end of the forward
+        start = first.astype(np.int64) - (np.cumsum(lens) - lens)  # position of a sequence's row r = start + r
+        return np.repeat(slots, lens), (np.arange(int(lens.sum())) + np.repeat(start, lens)).astype(np.int32)
+
+    def begin_ranges(self, seq_ids, append_lens):
+        """:meth:`begin_forward` for a caller that lays out the rows itself: per sequence its slot, its first position and the
+        number of tokens (arrays on the host)."""
         seq_ids = [int(s) for s in seq_ids]
         append_lens = [int(a) for a in append_lens]
         both = list(zip(seq_ids, append_lens))  # (what one of them has more of has no rows)
@@ -138,9 +149,7 @@ class PagedCache:
         finally:  # (sequences before one that finds no page keep what they got)
             self._push_pages(changed)
         self._pending = (seq_ids, append_lens)
-        lens = np.maximum(lens, 0)  # a negative length takes tokens back at the end of the forward
-        start = first.astype(np.int64) - (np.cumsum(lens) - lens)  # position of a sequence's row r = start + r
-        return np.repeat(slots, lens), (np.arange(int(lens.sum())) + np.repeat(start, lens)).astype(np.int32)
+        return slots, first, lens
 
     def end_forward(self):
         seq_ids, append_lens = self._pending

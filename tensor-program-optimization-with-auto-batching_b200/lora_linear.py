@@ -130,7 +130,12 @@ class MultiLoraLinear(nn.Module):
         cache = self._ctx.slot_cache if self._ctx is not None else None
         if cache is not None and key in cache:
             return cache[key]
-        t = torch.from_numpy(np.repeat(np.array(slots_per_batch_row, dtype=np.int32), per_row)).pin_memory().to(device, non_blocking=True)
+        values = np.array(slots_per_batch_row, dtype=np.int32)
+        if values.size <= ops.PUT_AT_MOST and per_row > 0:
+            t = torch.empty(values.size * per_row, dtype=torch.int32, device=device)
+            ops.put_i32(t, values, per_row)
+        else:
+            t = torch.from_numpy(np.repeat(values, per_row)).pin_memory().to(device, non_blocking=True)
         if cache is not None:
             if len(cache) > 64:
                 cache.clear()

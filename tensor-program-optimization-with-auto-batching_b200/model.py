@@ -311,7 +311,7 @@ class Engine(EngineBase):
         # prompt passes: tiles of <= 128 consecutive rows of one sequence for the tensor-core attention
         self.tc_prefill = os.environ.get("MLORA_TC_PREFILL", "1") != "0" and m.D == 128 and kv.page_size == 16
         self.pf_tiles = torch.zeros((T + 127) // 128 + kv.max_batch + 1, 4, dtype=torch.int32, device=dev)
-        self.pf_status = torch.zeros(1, dtype=torch.int32, device=dev)
+        self.pf_status = self._own_status_word()
         self._n_pf_tiles = 0
         self._graphs = {}
         self.fuse_norm_shrink = os.environ.get("MLORA_FUSE_NORM_SHRINK", "1") != "0"
@@ -464,11 +464,6 @@ class Engine(EngineBase):
 
     def _end_prompt_pass(self):
         self._n_pf_tiles = 0
-
-    def _check_prompt_status(self):
-        if int(self.pf_status.item()):
-            self.pf_status.zero_()
-            raise RuntimeError("mlora: the prompt attention kernel gave up a bounded wait; this pass's results are undefined")
 
     def forward(self, T: int, fused_append: bool, use_lora: bool = True, lm_rows=None, n_lm=None, hidden=None):
         """One pass over the T rows staged in self.tokens / self.slots / self.row_slot /

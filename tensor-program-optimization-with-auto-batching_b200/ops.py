@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes as C
 from dataclasses import dataclass
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -22,8 +23,8 @@ def _ptr(t):  # (plain numbers: the prototypes convert them)
     return None if t is None else t.data_ptr()
 
 
-def _stream():
-    return torch.cuda.current_stream().cuda_stream
+def _stream():  # (the handle alone: torch.cuda.current_stream() builds an object around it, 2 us of every launch)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def _need_cuda(*ts):
@@ -467,6 +468,22 @@ def paged_attention_shrink(qkv, k_pages, v_pages, block_table, row_slot, row_pos
         _ptr(stack.A_all), _ptr(stack.ranks), _ptr(slots), stack.A_all.shape[0], stack.r_max, _ptr(u), _ptr(work),
         work.numel(), _stream()), "mlora_paged_attention_shrink")
     return out
+
+
+PUT_AT_MOST = 1792  # values that travel in launch parameters (two launches); more go through pinned memory
+
+
+def put_i32(dst, values, repeat: int = 1):
+    """dst[i] = values[i // repeat]: a small host table (int32 array) into a contiguous device table, through launch parameters."""
+    values = np.ascontiguousarray(values, dtype=np.int32)
+    check(_lib.lib().mlora_put_i32(_ptr(dst), values.__array_interface__["data"][0], values.size, repeat, _stream()), "mlora_put_i32")
+
+
+def put_rows(seqs, slots, row_slot, row_pos):
+    """Row tables of a prompt pass from ``seqs`` int32 [n, 4]: cache slot, adapter slot, rows, position of the first row."""
+    seqs = np.ascontiguousarray(seqs, dtype=np.int32)
+    check(_lib.lib().mlora_put_rows(seqs.__array_interface__["data"][0], seqs.shape[0], _ptr(slots), _ptr(row_slot), _ptr(row_pos), _stream()),
+          "mlora_put_rows")
 
 
 def kv_begin_decode(row_slot, seq_lens, row_pos):
