@@ -476,12 +476,18 @@ PUT_AT_MOST = 1792  # values that travel in launch parameters (two launches); mo
 def put_i32(dst, values, repeat: int = 1):
     """dst[i] = values[i // repeat]: a small host table (int32 array) into a contiguous device table, through launch parameters."""
     values = np.ascontiguousarray(values, dtype=np.int32)
+    if dst.get_device() != torch.cuda.current_device():  # (a cache may be filled from another device, as with a copy)
+        with torch.cuda.device(dst.device):
+            return put_i32(dst, values, repeat)
     check(_lib.lib().mlora_put_i32(_ptr(dst), values.__array_interface__["data"][0], values.size, repeat, _stream()), "mlora_put_i32")
 
 
 def put_rows(seqs, slots, row_slot, row_pos):
     """Row tables of a prompt pass from ``seqs`` int32 [n, 4]: cache slot, adapter slot, rows, position of the first row."""
     seqs = np.ascontiguousarray(seqs, dtype=np.int32)
+    if slots.get_device() != torch.cuda.current_device():
+        with torch.cuda.device(slots.device):
+            return put_rows(seqs, slots, row_slot, row_pos)
     check(_lib.lib().mlora_put_rows(seqs.__array_interface__["data"][0], seqs.shape[0], _ptr(slots), _ptr(row_slot), _ptr(row_pos), _stream()),
           "mlora_put_rows")
 
