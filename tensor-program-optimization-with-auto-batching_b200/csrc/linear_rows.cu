@@ -227,6 +227,7 @@ __global__ void __launch_bounds__(rw_threads(LORA), 1) linear_rows_kernel(const 
             }
             break;
           }
+          __syncwarp();  // (the list as lane 0 has waited for it; a shuffle orders no memory)
           n_seg = s_nseg;
         }
         if (LORA && n_seg >= 0) {

@@ -58,3 +58,11 @@ def test_a_cta_of_a_pair_leaves_after_its_last_arrivals():
     builders = src[src.index("const uint32_t cache_lead"):src.index("__syncthreads();\n  if (s_abort)")]
     assert builders.index("++n_batch;") < builders.rindex("wait(cache_empty, (n_batch - 1) & 1);")
     assert builders.rindex("wait(cache_empty") > builders.rindex("mbar_arrive_cluster(cache_lead)")
+
+
+def test_lanes_read_behind_a_warp_barrier_what_one_lane_waited_for():
+    """A shuffle hands over the verdict of the waiting lane and orders no memory for the others."""
+    src = _source("linear_rows.cu")
+    copies = src[src.index("else if (warp < kRwProducts)") - 6000:src.index("else if (warp < kRwProducts)")]
+    wait = copies[copies.index("mbar_wait(list_bar"):]
+    assert "__syncwarp();" in wait[:wait.index("n_seg = s_nseg")].split("break;")[-1]
