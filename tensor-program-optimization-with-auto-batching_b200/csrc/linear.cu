@@ -123,14 +123,6 @@ static int linear_impl(const void* d_x, int64_t ldx, const void* d_W, void* d_y,
                                      const_cast<float*>(d_u), stream);
     if (rc != MLORA_OK) return rc;
   }
-  // Many distinct adapters on the kernel that takes B from its ring: no second launch, and y is rounded once.  us for all of
-  // a call, per-row expand behind that kernel against this: 16 adapters of rank 64, 16 rows 4096 -> 12288 28.8 / 25.1, 4096 -> 22016 SiLU*up
-  // 57.5 / 49.8; 32 of rank 16 4096 -> 12288 28.7 / 25.2; but 32 in front of SiLU*up 49.2 / 53.7 (rank 16), 83.8 / 91.5 (rank 64).
-  if ((flags & MLORA_LORA_PER_ROW) && d_u && !(flags & (MLORA_B_SPLIT | MLORA_FORCE_SIMT)) && d_work && linear_tc_supported(a) &&
-      (T <= 16 || !(flags & MLORA_SILU_MUL)) && linear_rows_chosen(a)) {
-    a.flags &= ~MLORA_LORA_PER_ROW;
-    return launch_linear_tc(a, d_work, work_bytes, st);
-  }
   if ((flags & MLORA_LORA_PER_ROW) && (flags & MLORA_SILU_MUL) && d_u && lora_expand_silu_supported(a) &&
       work_bytes >= mlora_linear_workspace_flags(T, in, out, flags) && d_work) {
     // many distinct adapters in front of SiLU*up: the projection writes fp32 pre-activations of the interleaved gate / up

@@ -92,3 +92,35 @@ def test_rotary(cuda, Hq, Hkv, ps, fused):
     assert torch.equal(live, ~torch.isnan(got[0][0])) and float(((k0 - k1).abs() - 2 ** -7 * k1.abs()).max()) <= 0 and int((k0 != k1).sum()) < T * Hkv
     assert torch.equal(got[0][1].view(torch.int16), got[1][1].view(torch.int16))
     _same(got[0][2], got[1][2])
+
+
+@pytest.mark.parametrize("Hq,Hkv,ps", [(32, 8, 16), (32, 16, 32), (32, 8, 32), (32, 16, 16)])
+@pytest.mark.parametrize("n_splits", [1, 3])
+def test_keys_with_a_score_of_minus_infinity(cuda, Hq, Hkv, ps, n_splits):
+    """They are left out, whatever their value is, for the heads that score them so; a row of nothing else (or of no scores at all) is zero."""
+    ops = load("ops")
+    lens = [LENS[i % len(LENS)] for i in range(18)]
+    T, D = len(lens), 128
+    r, K, V, bt, rs, rp = _case(cuda, T, Hq, Hkv, ps, lens, Hq + ps + 1)
+    q = r(T, Hq, D).bfloat16()
+    q[:, ::2, 5], q[:, 1::2, 5] = 1.0, 0.25  # (both heads of a pair see column 5 with a plus sign)
+    q[:, :, 6] = 0.0
+    q = q.view(T, Hq * D)
+    for t, n in enumerate(lens):
+        for key in range(n + 1):
+            if (n > 200 and key % 5 == 3) or n in (15, 33, 64) or (n == 100 and key < 40):
+                K[bt[t, key // ps], :, key % ps, 5] = float("-inf")
+                V[bt[t, key // ps], :, key % ps] = float("inf") if key % 2 else float("nan")
+            if n == 17:
+                K[bt[t, key // ps], :, key % ps, 6] = float("nan")
+    out, one = torch.zeros_like(q), torch.zeros_like(q)
+
+    def run(rows, o):
+        w = torch.zeros(max(ops.paged_attention_workspace(T, Hq, D, n_splits), 16), dtype=torch.uint8, device=cuda)
+        ops.paged_attention_masked(q[rows], K, V, bt, rs[rows], rp[rows], Hq, D ** -0.5, o[rows], n_splits=n_splits, work=w)
+
+    run(slice(0, T), out)
+    for t in range(T):
+        run(slice(t, t + 1), one)
+    _same(out, one)
+    assert all(bool((out[t] == 0).all()) == (n in (15, 17, 33, 64)) for t, n in enumerate(lens))
