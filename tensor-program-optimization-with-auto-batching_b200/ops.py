@@ -473,9 +473,22 @@ def paged_attention_shrink(qkv, k_pages, v_pages, block_table, row_slot, row_pos
 PUT_AT_MOST = 1792  # values that travel in launch parameters (two launches); more go through pinned memory
 
 
+def _room_for(n, *tables):
+    """The launches know no length: a table that is too small is refused here, as a copy would refuse it."""
+    for t in tables:
+        if t.dtype != torch.int32 or not t.is_contiguous():
+            raise ValueError("mlora: tables on the device are contiguous int32")
+        if n > t.numel():
+            raise RuntimeError(f"mlora: {n} values into a table of {t.numel()}")
+
+
 def put_i32(dst, values, repeat: int = 1):
     """dst[i] = values[i // repeat]: a small host table (int32 array) into a contiguous device table, through launch parameters."""
     values = np.ascontiguousarray(values, dtype=np.int32)
+    _room_for(values.size * repeat, dst)
+    if not values.size:
+        return
+    _need_cuda(dst)
     if dst.get_device() != torch.cuda.current_device():  # (a cache may be filled from another device, as with a copy)
         with torch.cuda.device(dst.device):
             return put_i32(dst, values, repeat)
@@ -485,6 +498,13 @@ def put_i32(dst, values, repeat: int = 1):
 def put_rows(seqs, slots, row_slot, row_pos):
     """Row tables of a prompt pass from ``seqs`` int32 [n, 4]: cache slot, adapter slot, rows, position of the first row."""
     seqs = np.ascontiguousarray(seqs, dtype=np.int32)
+    if seqs.ndim != 2 or seqs.shape[1] != 4:
+        raise ValueError("mlora.put_rows: four numbers per sequence")
+    rows = int(seqs[:, 2].sum(dtype=np.int64))
+    _room_for(rows, slots, row_slot, row_pos)
+    if not seqs[:, 2].any():
+        return
+    _need_cuda(slots, row_slot, row_pos)
     if slots.get_device() != torch.cuda.current_device():
         with torch.cuda.device(slots.device):
             return put_rows(seqs, slots, row_slot, row_pos)
