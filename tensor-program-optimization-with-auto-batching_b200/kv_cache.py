@@ -56,7 +56,10 @@ class PagedCache:
         self._slot_of[sid] = slot
         self._n_pages_of[sid] = 0
         self._len_host[slot] = 0
-        self._push(self.seq_lens[slot:slot + 1], self._len_host[slot:slot + 1])
+        if self.seq_lens.is_cuda:
+            self._push(self.seq_lens[slot:slot + 1], self._len_host[slot:slot + 1])
+        else:
+            self.seq_lens[slot] = 0
         return slot
 
     def _push(self, dst, src_np):

@@ -67,3 +67,13 @@ def test_adapter_slots_beyond_32_bits_are_refused(slot):
     with pytest.raises(OverflowError):
         eng.extend([4], [[1, 2, 3]], [slot])
     assert eng.kv.tokens_reserved(4) == 0
+
+
+def test_sequences_of_a_cache_without_a_gpu():
+    """Adding a sequence clears its length in place: no pinned memory, which a machine without a GPU does not have."""
+    kv = load("kv_cache").PagedCache(3, 96, 64, 16, "cpu")
+    kv.seq_lens.fill_(7)
+    assert [kv.seq_lens[kv.add_sequence(s)].item() for s in (5, 9)] == [0, 0]
+    assert kv.seq_lens.sum().item() == 7
+    kv.remove_sequence(5)
+    assert kv.slot(9) == 1
