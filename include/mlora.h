@@ -144,7 +144,11 @@ int mlora_lora_shrink(const void* d_x, int64_t ldx, const void* d_A_all, const i
  *   MMA issuer waiting for the operand cache, 7 (128) finishing CTA waiting for the partial sums of a
  *   split tile.  The output of that call is then undefined, and because late contributors of a split
  *   tile may still bump its arrival counter afterwards, the whole buffer must be zero-filled again
- *   before its next use (the word is sticky: the caller clears it). */
+ *   before its next use (the word is sticky: the caller clears it).
+ *   The MLORA_WORK_CALLER_BYTES at MLORA_WORK_CALLER_OFFSET are the caller's: no kernel of this library that is given the
+ *   buffer as scratch touches them (the engines keep the status word of their attention kernels there). */
+#define MLORA_WORK_CALLER_OFFSET 240
+#define MLORA_WORK_CALLER_BYTES 16
 size_t mlora_linear_workspace(int32_t T, int32_t in, int32_t out);
 /* Introspection, host side only (no device work): how the one-CTA tensor-core kernel deals a projection of this shape to its
  * CTAs.  (Batches of more than 128 rows whose tiles fill the GPU run on pairs of CTAs instead, with tiles of 256 outputs.)

@@ -37,7 +37,8 @@ constexpr int kMaxGrid = 256;
 constexpr int kHeaderBytes = 256;
 constexpr int kExitOffset = 8;
 constexpr int kBarOffset = 64;
-static_assert(kBarOffset + kMaxPhases * kBarsPerPhase * 4 <= kHeaderBytes, "barriers must fit the header");
+static_assert(kBarOffset + kMaxPhases * kBarsPerPhase * 4 <= MLORA_WORK_CALLER_OFFSET, "barriers must fit the header, in front of the caller's bytes");
+static_assert(MLORA_WORK_CALLER_OFFSET + MLORA_WORK_CALLER_BYTES <= kHeaderBytes, "the caller's bytes are in the header");
 
 enum : int { kStWProducer = 1, kStMma = 2, kStEpilogue = 4, kStAcc = 8, kStXProducer = 16, kStBuilder = 32,
              kStCache = 64, kStPartials = 128, kStGridBarrier = 256 };

@@ -37,7 +37,8 @@ constexpr int BM = 128;            // weight rows per tile (MMA M)
 constexpr int kThreads = 224;          // 7 warps: W producer, MMA, 4 epilogue, x producer
 #define kPrefetch p.prefetch          // weight tiles requested from HBM into L2 ahead of the ring
 constexpr int kEpiThreads = 128;
-constexpr int kHeaderBytes = 256;  // status word + padding at the start of the scratch buffer
+constexpr int kHeaderBytes = 256;  // status word, padding, the caller's bytes at the start of the scratch buffer
+static_assert(MLORA_WORK_CALLER_OFFSET >= 4 && MLORA_WORK_CALLER_OFFSET + MLORA_WORK_CALLER_BYTES <= kHeaderBytes, "the caller's bytes are in the header");
 constexpr int kMaxGrid = 256;      // tickets / partial slots are sized for at most this many CTAs
 constexpr int kStageUMax = 8 * 1024;  // shrink outputs are staged in shared memory up to this size
 

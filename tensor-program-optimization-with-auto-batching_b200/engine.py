@@ -33,7 +33,8 @@ class EngineBase:
     adapter slots, ``row_slot`` = cache slots, ``row_pos``), returning (logits, next tokens);
     ``_begin_prompt_pass(chunk)`` / ``_end_prompt_pass()`` around the forward of a prompt pass, ``chunk`` a list of
     (sequence id, first row, rows, position of the first row);
-    kernels with bounded waits report to ``_own_status_word()``."""
+    kernels with bounded waits report to ``_own_status_word()``; what an engine checks beyond that after the last pass of
+    a call: ``_check_prompt_status()``."""
 
     def __init__(self, model, kv: PagedCache, max_rows: int):
         self.m, self.kv, self.max_rows = model, kv, int(max_rows)
@@ -60,28 +61,29 @@ class EngineBase:
     def _end_prompt_pass(self):
         pass
 
+    def _check_prompt_status(self):
+        pass
+
     def status_word(self) -> int:
         """Status word of the projection kernels' scratch (synchronises): non-zero after a bounded wait expired
         somewhere since the buffer was last cleared; the outputs since then are undefined."""
         return ops.status_word(self.ws_linear)
 
     def _own_status_word(self):
-        """A word of the projection scratch's header that no projection uses, for the engine's other kernels with bounded waits:
+        """The word of the projection scratch's header that is the caller's, for the engine's other kernels with bounded waits:
         :meth:`check_status` reads both words at once."""
-        return self.ws_linear[240:244].view(torch.int32)
+        return self.ws_linear[ops.WORK_CALLER_OFFSET:ops.WORK_CALLER_OFFSET + 4].view(torch.int32)
 
     def check_status(self):
         """Raises if a kernel gave up a bounded wait, after re-zeroing the scratch (arrival counters of split tiles may be stale
         after such a failure) so that the engine stays usable."""
-        words = self.ws_linear[:244].view(torch.int32).tolist()
-        st, own = words[0], words[60]
-        if st or own:
-            self.ws_linear.zero_()
-        if st:
-            raise RuntimeError(f"mlora: a projection kernel gave up a bounded wait (status bits {st:#x}); "
-                               "the results of this pass are undefined")
-        if own:
-            raise RuntimeError("mlora: an attention kernel gave up a bounded wait; this pass's results are undefined")
+        words = self.ws_linear[:ops.WORK_CALLER_OFFSET + 4].view(torch.int32).tolist()
+        st, own = words[0], words[-1]
+        if not st and not own:
+            return
+        self.ws_linear.zero_()
+        who = ([f"a projection kernel (status bits {st:#x})"] if st else []) + (["an attention kernel"] if own else [])
+        raise RuntimeError(f"mlora: {' and '.join(who)} gave up a bounded wait; the results of this pass are undefined")
 
     def _stage(self, dst, values, dtype):
         t = torch.as_tensor(np.asarray(values), dtype=dtype)
@@ -170,6 +172,7 @@ class EngineBase:
             kv.end_forward()
             self._end_prompt_pass()
         self.check_status()  # (synchronises; prefill is not the latency-critical call)
+        self._check_prompt_status()
         return out_logits, out_tok
 
     def prefill(self, seq_ids, prompts, adapter_slots, use_lora=True):

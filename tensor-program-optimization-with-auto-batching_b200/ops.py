@@ -59,6 +59,9 @@ def new_workspace(nbytes: int, device):
     return torch.zeros(max(int(nbytes), 256), dtype=torch.uint8, device=device)
 
 
+WORK_CALLER_OFFSET = 240  # bytes of a projection scratch that are the caller's: MLORA_WORK_CALLER_OFFSET
+
+
 def status_word(work) -> int:
     """The status word at the start of a projection scratch buffer (0 = no bounded wait ever expired)."""
     return int(work[:4].view(torch.int32).item())
