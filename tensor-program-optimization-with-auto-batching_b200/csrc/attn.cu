@@ -70,6 +70,12 @@ __device__ __forceinline__ float rope_inv_freq(float theta, int i, int D) {
   return powf(theta, -(float)(2 * i) / (float)D);
 }
 
+// A pair of columns turned by an angle.  Which product is rounded first is written down: the compiler chose it kernel by kernel, and the
+// key that is cached for a token must not depend on the kernel that appends it.
+__device__ __forceinline__ float2 rotate_pair(float x1, float x2, float sn, float cs) {
+  return make_float2(fmaf(x1, cs, -__fmul_rn(x2, sn)), fmaf(x2, cs, __fmul_rn(x1, sn)));
+}
+
 __device__ __forceinline__ void merge_state(float& m, float& l, float (&acc)[8], float mo, float lo,
                                             const float (&acco)[8]) {
   const float mn = fmaxf(m, mo);
@@ -152,8 +158,8 @@ __global__ void __launch_bounds__(128) paged_attn_kernel(AttnArgs a) {
     if (a.fused) {
       float sn, cs;
       sincosf((float)pos * rope_inv_freq(a.theta, i, D), &sn, &cs);
-      const float r1 = q1 * cs - q2 * sn, r2 = q2 * cs + q1 * sn;
-      q1 = r1, q2 = r2;
+      const float2 r = rotate_pair(q1, q2, sn, cs);
+      q1 = r.x, q2 = r.y;
     }
     sq[i] = q1 * qscale;
     sq[i + D / 2] = q2 * qscale;
@@ -163,7 +169,8 @@ __global__ void __launch_bounds__(128) paged_attn_kernel(AttnArgs a) {
     const float k1 = __bfloat162float(kr[i]), k2 = __bfloat162float(kr[i + D / 2]);
     float sn, cs;
     sincosf((float)pos * rope_inv_freq(a.theta, i, D), &sn, &cs);
-    const bf16 r1 = __float2bfloat16_rn(k1 * cs - k2 * sn), r2 = __float2bfloat16_rn(k2 * cs + k1 * sn);
+    const float2 r = rotate_pair(k1, k2, sn, cs);
+    const bf16 r1 = __float2bfloat16_rn(r.x), r2 = __float2bfloat16_rn(r.y);
     sk[i] = __bfloat162float(r1);
     sk[i + D / 2] = __bfloat162float(r2);
     if (h % rep == 0 && can_store) {
@@ -489,13 +496,15 @@ __global__ void __launch_bounds__(128, REP == 4 ? 2 : 4) paged_attn_group_kernel
 #pragma unroll
         for (int j = 0; j < REP; ++j) {
           const float q1 = __bfloat162float(row[(h0 + j) * D + i]), q2 = __bfloat162float(row[(h0 + j) * D + i + D / 2]);
-          sq[j][i] = (a.fused ? q1 * cs - q2 * sn : q1) * a.qscale;
-          sq[j][i + D / 2] = (a.fused ? q2 * cs + q1 * sn : q2) * a.qscale;
+          const float2 r = a.fused ? rotate_pair(q1, q2, sn, cs) : make_float2(q1, q2);
+          sq[j][i] = r.x * a.qscale;
+          sq[j][i + D / 2] = r.y * a.qscale;
         }
         if (has_new) {
           const bf16* kr = row + (size_t)(a.Hq + kvh) * D;
           const float k1 = __bfloat162float(kr[i]), k2 = __bfloat162float(kr[i + D / 2]);
-          const bf16 r1 = __float2bfloat16_rn(k1 * cs - k2 * sn), r2 = __float2bfloat16_rn(k2 * cs + k1 * sn);
+          const float2 r = rotate_pair(k1, k2, sn, cs);
+          const bf16 r1 = __float2bfloat16_rn(r.x), r2 = __float2bfloat16_rn(r.y);
           sk[i] = __bfloat162float(r1);
           sk[i + D / 2] = __bfloat162float(r2);
           if (stores) {
@@ -751,11 +760,8 @@ __global__ void __launch_bounds__(256) kv_append_rope_kernel(bf16* __restrict__ 
     const __nv_bfloat162 b = *reinterpret_cast<const __nv_bfloat162*>(p + i + half);
     const float x1a = __bfloat162float(a.x), x1b = __bfloat162float(a.y);
     const float x2a = __bfloat162float(b.x), x2b = __bfloat162float(b.y);
-    __nv_bfloat162 r1, r2;
-    r1.x = __float2bfloat16_rn(x1a * cs0 - x2a * sn0);
-    r1.y = __float2bfloat16_rn(x1b * cs1 - x2b * sn1);
-    r2.x = __float2bfloat16_rn(x2a * cs0 + x1a * sn0);
-    r2.y = __float2bfloat16_rn(x2b * cs1 + x1b * sn1);
+    const float2 ra = rotate_pair(x1a, x2a, sn0, cs0), rb = rotate_pair(x1b, x2b, sn1, cs1);
+    const __nv_bfloat162 r1 = __floats2bfloat162_rn(ra.x, rb.x), r2 = __floats2bfloat162_rn(ra.y, rb.y);
     bf16* dst = head < Hq ? p : k_pages + (((size_t)page * Hkv + (head - Hq)) * PS + pos % PS) * D;
     *reinterpret_cast<__nv_bfloat162*>(dst + i) = r1;
     *reinterpret_cast<__nv_bfloat162*>(dst + i + half) = r2;
@@ -768,7 +774,7 @@ __global__ void __launch_bounds__(256) kv_append_rope_kernel(bf16* __restrict__ 
   }
 }
 
-// The same rotation (in fp32; a last bit may differ) in 16-byte pieces, where the key pages are aligned to that: a thread takes 8 dimensions of the first half of a
+// The same rotation in 16-byte pieces, where the key pages are aligned to that: a thread takes 8 dimensions of the first half of a
 // head and the 8 that rotate with them, and requests its pieces of two heads and of two value heads before it waits for the
 // row's sines and cosines (computed once per row, not once per thread) and its page.  Bound by HBM: a row is read and
 // written once.  Measured, 8192 rows, 32 + 2 x 32 heads of 128: 108 -> 80 us (403 MB, 5.0 TB/s); 1000 rows of 40 heads 17.9 -> 14.6.
@@ -818,9 +824,9 @@ __global__ void __launch_bounds__(kRope16Threads) kv_append_rope16_kernel(bf16* 
         unpack8(hi[b], x2);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const float sn = s_sn[i + e], cs = s_cs[i + e];
-          r1[e] = x1[e] * cs - x2[e] * sn;
-          r2[e] = x2[e] * cs + x1[e] * sn;
+          const float2 r = rotate_pair(x1[e], x2[e], s_sn[i + e], s_cs[i + e]);
+          r1[e] = r.x;
+          r2[e] = r.y;
         }
         bf16* dst = (head < Hq ? row + (size_t)head * D : k_pages + (((size_t)page * Hkv + (head - Hq)) * PS + pos % PS) * D) + i;
         *reinterpret_cast<uint4*>(dst) = pack8(r1);

@@ -48,3 +48,24 @@ def test_heads_and_key_page_alignment(Hq, Hkv, D, page):
         assert torch.equal(v[at[live], :, in_page[live]], qkv.view(T, -1, D)[live][:, Hq + Hkv:])
         assert torch.equal(rows[~live], qkv[~live]) and torch.equal(rows.view(T, -1, D)[:, Hq:], qkv.view(T, -1, D)[:, Hq:])
         assert (k.transpose(1, 2)[~written] == 7).all() and (v.transpose(1, 2)[~written] == 7).all()
+
+
+def test_the_same_key_whoever_appends_it():
+    """Decode of single heads, of four and of two that share a key head, and both kernels for prompt rows."""
+    ops = load("ops")
+    T, Hkv, D, page, theta = 1024, 8, 128, 16, 10000.0
+    g = torch.Generator(device="cuda").manual_seed(3)
+    kv = torch.randn(T, 2 * Hkv * D, generator=g, device="cuda").bfloat16()
+    pos = torch.randint(0, 200 * page, (T,), generator=g, device="cuda").to(torch.int32)
+    table = torch.arange(T, device="cuda", dtype=torch.int32)[:, None].repeat(1, 200)  # (a row sees its own page alone)
+    slot, at, got = torch.arange(T, device="cuda", dtype=torch.int32), torch.arange(T, device="cuda"), []
+    for Hq, off in ((8, 0), (32, 0), (16, 0), (8, None), (8, 2)):
+        rows = torch.cat([torch.randn(T, Hq * D, generator=g, device="cuda").bfloat16(), kv], 1)
+        n, v = T * Hkv * page * D, torch.zeros(T, Hkv, page, D, device="cuda").bfloat16()
+        k = torch.zeros(n + 8, device="cuda").bfloat16()[off or 0:(off or 0) + n].view(T, Hkv, page, D)
+        if got and Hq == 8:
+            ops.kv_append_rope(rows, k, v, table, slot, pos, Hq, Hkv, D, page, theta)
+        else:
+            ops.paged_attention(rows, k, v, table, slot, pos, Hq, Hkv, D, page, theta, True, n_splits=1)
+        got.append(k[at, :, (pos % page).long()].view(torch.int16))
+    assert all(torch.equal(k, got[0]) for k in got)

@@ -86,10 +86,7 @@ def test_rotary(cuda, Hq, Hkv, ps, fused):
         for s in rows:
             ops.paged_attention(x[s], k, v, bt, rs[s], rp[s], Hq, Hkv, 128, ps, 10000.0, fused, out=o[s], n_splits=1)
         got.append((k, v, o))
-    # appended keys: the compiler may fuse the rotation's products the other way round, neighbouring bf16 values at most; values the same
-    live = ~torch.isnan(got[1][0])
-    k0, k1 = got[0][0][live].float(), got[1][0][live].float()
-    assert torch.equal(live, ~torch.isnan(got[0][0])) and float(((k0 - k1).abs() - 2 ** -7 * k1.abs()).max()) <= 0 and int((k0 != k1).sum()) < T * Hkv
+    assert torch.equal(got[0][0].view(torch.int16), got[1][0].view(torch.int16))  # what is appended: the same bits
     assert torch.equal(got[0][1].view(torch.int16), got[1][1].view(torch.int16))
     _same(got[0][2], got[1][2])
 
