@@ -62,9 +62,10 @@ extern "C" {
                                front of a discrete choice (an expert router picks the largest of its scores): there
                                another order of fp32 sums is another choice at a near tie */
 #define MLORA_ANY_SUMS 2048 /* the caller does not need the sums over `in` in the order of mlora_linear_plan: up to 32 rows of
-                               a packed weight may run on the kernel that gives every CTA whole output rows.  Without this
-                               flag, or with MLORA_STABLE_SUMS, a call keeps the plan's sums, whose bits
-                               mlora_decode_chain reproduces */
+                               a packed weight may run on the kernel that gives every CTA whole output rows.  Which kernel that
+                               is changes with the rows (1..4, 5..16, 17..32), `in` and `out` (mlora_linear_rows_plan), so a
+                               row's last bits may depend on the size of its batch.  Without this flag, or with
+                               MLORA_STABLE_SUMS, a call keeps the plan's sums, whose bits mlora_decode_chain reproduces */
 
 int mlora_version(void);
 const char* mlora_last_error(void);
@@ -165,6 +166,12 @@ int mlora_linear_plan(int32_t T, int32_t in, int32_t out, int32_t* h_plan12);
  * pair w takes (row pair, token tile) number w, w + [1], ..., row pair major. */
 int mlora_linear_pair_plan(int32_t T, int32_t in, int32_t out, int32_t r_max, int32_t n_mod, const int32_t* h_mod_offsets,
                            int32_t flags, int32_t* h_plan6);
+/* ... and whether a call runs with whole output rows per CTA (MLORA_ANY_SUMS), and how (host side only; arguments as above, x, u
+ * and y aligned as that kernel wants them).  h_plan6 (HOST, 6 int32): [0] passes over x (0: the call runs on another kernel, the
+ * rest is 0 too), [1] CTAs, [2] row groups (8 outputs) of a CTA's widest pass, [3] row groups it multiplies, [4] k-blocks (64 of
+ * in) per ring slot, [5] ring slots. */
+int mlora_linear_rows_plan(int32_t T, int32_t in, int32_t out, int32_t r_max, int32_t n_mod, const int32_t* h_mod_offsets,
+                           int32_t flags, int32_t* h_plan6);
 /* The same for a call with these flags: more than mlora_linear_workspace only for MLORA_SILU_MUL | MLORA_LORA_PER_ROW. */
 size_t mlora_linear_workspace_flags(int32_t T, int32_t in, int32_t out, int32_t flags);
 /* Weight pre-packing (load time).  Rewrites W [out,in] bf16 as tiles [ceil(out/128)][ceil(in/64)] of
@@ -228,7 +235,7 @@ int mlora_lora_linear(const void* d_x, int64_t ldx, const void* d_W, void* d_y, 
  * i+1 = d_y of phase i, or d_delta of phase i+1 = d_y of phase i when it has a norm); the kernel orders
  * them with grid-wide barriers instead of kernel boundaries and keeps streaming weights across them.
  * Results are bit-identical to the same sequence of mlora_residual_rmsnorm / mlora_lora_shrink /
- * mlora_linear calls (same tile split, same reduction orders).
+ * mlora_linear calls without MLORA_ANY_SUMS (same tile split, same reduction orders).
  *   d_x [T,in] bf16 (row stride ldx; written by the norm when d_res != NULL, then ldx == in, in <= 8192)
  *   d_Wp: mlora_pack_weight layout.  d_y [T, out or out/2] bf16 (f32 with MLORA_OUT_F32), rows 16-byte multiples
  *   flags: MLORA_OUT_F32 | MLORA_SILU_MUL only

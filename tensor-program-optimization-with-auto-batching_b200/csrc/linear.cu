@@ -32,6 +32,26 @@ extern "C" int mlora_linear_pair_plan(int32_t T, int32_t in, int32_t out, int32_
   return MLORA_OK;
 }
 
+extern "C" int mlora_linear_rows_plan(int32_t T, int32_t in, int32_t out, int32_t r_max, int32_t n_mod,
+                                      const int32_t* h_mod_offsets, int32_t flags, int32_t* h_plan6) {
+  MLORA_REQUIRE(T > 0 && in > 0 && out > 0 && r_max >= 0 && n_mod >= 1 && n_mod <= 8 && (n_mod == 1 || h_mod_offsets || (flags & MLORA_SILU_MUL)) && h_plan6,
+                "linear_rows_plan: bad arguments");
+  const bool silu = (flags & MLORA_SILU_MUL) != 0;
+  LinearArgs a{};
+  a.T = T;
+  a.in = in;
+  a.out = out;
+  a.flags = flags;
+  alignas(16) static const float some = 0.f;  // (only whether there are shrink outputs counts)
+  a.u = r_max ? &some : nullptr;
+  a.r_max = silu ? 2 * r_max : r_max;
+  a.n_mod = silu ? 1 : n_mod;
+  for (int m = 0; m <= a.n_mod && a.n_mod > 1; ++m) a.mod_off[m] = h_mod_offsets[m];
+  for (int i = 0; i < 6; ++i) h_plan6[i] = 0;
+  if (linear_rows_chosen(a)) linear_rows_plan(a, h_plan6);
+  return MLORA_OK;
+}
+
 static size_t pre_offset(int32_t T, int32_t in, int32_t out) { return (linear_tc_workspace(T, in, out) + 255) & ~(size_t)255; }
 
 extern "C" size_t mlora_linear_workspace_flags(int32_t T, int32_t in, int32_t out, int32_t flags) {

@@ -136,6 +136,7 @@ void linear_tc_plan(int T, int in, int out, int32_t* v12);
 int launch_linear_tc(const LinearArgs& a, void* work, size_t work_bytes, cudaStream_t st);
 // The same with whole output rows per CTA, for up to 32 rows whose sums may be taken in any order (of `work` only the status word).
 bool linear_rows_chosen(const LinearArgs& a);
+void linear_rows_plan(const LinearArgs& a, int32_t* v6);
 int launch_linear_rows(const LinearArgs& a, void* work, cudaStream_t st);
 // The same on pairs of CTAs, for prompt-size batches (likewise).
 bool linear_pair_supported(const LinearArgs& a);

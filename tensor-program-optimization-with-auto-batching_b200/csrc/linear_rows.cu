@@ -525,44 +525,80 @@ int launch_rows(const CUtensorMap& mx, const RwParams& p, int grid, cudaStream_t
   return MLORA_OK;
 }
 
+struct RowsPlan {
+  int units, unit, grid, passes;
+  int groups, pairs;  // row groups of the widest pass; half of those that are multiplied (NP)
+  int kj, slot_bytes, slots;
+};
+
+// Row groups of a pass -> NP.  A pass multiplies 2 NP groups whatever it has, so the steps lie at widths that occur: over 148 SMs 4096
+// outputs have 4 groups, 5120 5, 12288 11, 15360 13, 22016 behind SiLU 20 (in two passes beyond 16 rows: 10).  A width in between
+// multiplies up to five groups for nothing.
+template <int XR>
+int np_for(int groups) {
+  constexpr int steps16[] = {2, 4, 6, 7, 10}, steps32[] = {2, 4, 5, 6};
+  if constexpr (XR > 16) {
+    for (int np : steps32)
+      if (groups <= 2 * np) return np;
+  } else {
+    for (int np : steps16)
+      if (groups <= 2 * np) return np;
+  }
+  return 0;
+}
+
+template <int XR>
+RowsPlan rows_plan(const LinearArgs& a, bool lora) {
+  using C = RwCfg<XR>;
+  RowsPlan q{};
+  const int k_blocks = (a.in + BK - 1) / BK;
+  q.unit = (a.flags & MLORA_SILU_MUL) ? 2 : 1;
+  q.units = (a.out + 8 * q.unit - 1) / (8 * q.unit);
+  q.grid = q.units < sm_count() ? q.units : sm_count();
+  const int most = (q.units + q.grid - 1) / q.grid, cap = C::kMaxG / q.unit;
+  q.passes = (most + cap - 1) / cap;
+  q.groups = (most + q.passes - 1) / q.passes * q.unit;
+  q.pairs = np_for<XR>(q.groups);
+  const int kb_bytes = q.groups * 1024 + C::kXBytes, ring = C::ring(lora);
+  // As many k-blocks per slot as leave four slots: a slot's hand-over costs its warps about 0.15 us whatever it holds (1 row,
+  // 11008 -> 4096: 27.6 us with two k-blocks per slot, 22 with eight).
+  q.kj = 4;
+  while (q.kj > 1 && (ring / (2 * q.kj * kb_bytes) < 4 || q.kj >= k_blocks)) q.kj >>= 1;
+  q.slot_bytes = 2 * q.kj * kb_bytes;
+  q.slots = ring / q.slot_bytes;
+  if (q.slots > kRwMaxSlots) q.slots = kRwMaxSlots;
+  return q;
+}
+
 template <int XR, bool LORA>
 int plan_rows(const LinearArgs& a, void* work, cudaStream_t st) {
-  using C = RwCfg<XR>;
   CUtensorMap mx;
   const int rc = make_map(&mx, a.x, a.T, a.in, a.ldx, XR);
   if (rc) return rc;
+  const RowsPlan q = rows_plan<XR>(a, LORA);
   RwParams p;
   p.a = a;
   p.k_blocks = (a.in + BK - 1) / BK;
   p.row_tiles = (a.out + BM - 1) / BM;
-  p.unit = (a.flags & MLORA_SILU_MUL) ? 2 : 1;
-  p.units = (a.out + 8 * p.unit - 1) / (8 * p.unit);
-  const int grid = p.units < sm_count() ? p.units : sm_count();
-  const int most = (p.units + grid - 1) / grid, cap = C::kMaxG / p.unit;
-  p.passes = (most + cap - 1) / cap;
-  const int kb_bytes = (most + p.passes - 1) / p.passes * p.unit * 1024 + C::kXBytes;
-  // As many k-blocks per slot as leave four slots: a slot's hand-over costs its warps about 0.15 us whatever it holds (1 row,
-  // 11008 -> 4096: 27.6 us with two k-blocks per slot, 22 with eight).
-  p.kj = 4;
-  while (p.kj > 1 && (C::ring(LORA) / (2 * p.kj * kb_bytes) < 4 || p.kj >= p.k_blocks)) p.kj >>= 1;
-  p.slot_bytes = 2 * p.kj * kb_bytes;
-  p.slots = C::ring(LORA) / p.slot_bytes;
-  if (p.slots > kRwMaxSlots) p.slots = kRwMaxSlots;
+  p.unit = q.unit;
+  p.units = q.units;
+  p.passes = q.passes;
+  p.kj = q.kj;
+  p.slot_bytes = q.slot_bytes;
+  p.slots = q.slots;
   p.lora_sub = a.r_max > 0 && a.r_max < 64 ? a.r_max : 64;
   p.n_sub = a.r_max > 64 ? a.r_max / 64 : 1;
   const int es = (a.flags & MLORA_OUT_F32) ? 4 : 2;
   p.vec = (reinterpret_cast<uintptr_t>(a.y) % (4 * es)) == 0 && a.ldy % 4 == 0;
   p.status = (int32_t*)work;
-  const int ng = (most + p.passes - 1) / p.passes * p.unit;  // the widest pass
-  if (ng <= 4) return launch_rows<XR, 2, LORA>(mx, p, grid, st);
-  if (ng <= 8) return launch_rows<XR, 4, LORA>(mx, p, grid, st);
+  if (q.pairs == 2) return launch_rows<XR, 2, LORA>(mx, p, q.grid, st);
+  if (q.pairs == 4) return launch_rows<XR, 4, LORA>(mx, p, q.grid, st);
+  if (q.pairs == 6) return launch_rows<XR, 6, LORA>(mx, p, q.grid, st);
   if constexpr (XR > 16) {
-    if (ng <= 10) return launch_rows<XR, 5, LORA>(mx, p, grid, st);
-    return launch_rows<XR, 6, LORA>(mx, p, grid, st);
+    return launch_rows<XR, 5, LORA>(mx, p, q.grid, st);
   } else {
-    if (ng <= 12) return launch_rows<XR, 6, LORA>(mx, p, grid, st);
-    if (ng <= 14) return launch_rows<XR, 7, LORA>(mx, p, grid, st);
-    return launch_rows<XR, 10, LORA>(mx, p, grid, st);
+    if (q.pairs == 7) return launch_rows<XR, 7, LORA>(mx, p, q.grid, st);
+    return launch_rows<XR, 10, LORA>(mx, p, q.grid, st);
   }
 }
 
@@ -589,6 +625,16 @@ bool linear_rows_chosen(const LinearArgs& a) {
 int launch_linear_rows(const LinearArgs& a, void* work, cudaStream_t st) {
   if (a.u == nullptr) return a.T <= 16 ? plan_rows<16, false>(a, work, st) : plan_rows<32, false>(a, work, st);
   return a.T <= 16 ? plan_rows<16, true>(a, work, st) : plan_rows<32, true>(a, work, st);
+}
+
+void linear_rows_plan(const LinearArgs& a, int32_t* v6) {
+  const RowsPlan q = a.T <= 16 ? rows_plan<16>(a, a.u != nullptr) : rows_plan<32>(a, a.u != nullptr);
+  v6[0] = q.passes;
+  v6[1] = q.grid;
+  v6[2] = q.groups;
+  v6[3] = 2 * q.pairs;
+  v6[4] = 2 * q.kj;
+  v6[5] = q.slots;
 }
 
 }  // namespace mlora

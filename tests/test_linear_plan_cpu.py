@@ -142,3 +142,58 @@ def test_stable_sums_take_pairs_only_where_no_tile_is_split(T, K, N):
     whole = p["gt"] > 0 or p["per_cta"] % p["k_blocks"] == 0
     stable = load("ops").STABLE_SUMS
     assert (_pair_plan(T, K, N, flags=stable)["bn"] > 0) == (whole and _pair_plan(T, K, N)["bn"] > 0)
+
+
+def _rows_plan(T, K, N, flags, mods=None, rank=0):
+    lib, ops = load("_lib").lib(), load("ops")
+    v, offs = (C.c_int32 * 6)(), (C.c_int32 * len(mods))(*mods) if mods else None
+    n_mod = len(mods) - 1 if mods else 2 if flags & ops.SILU_MUL and rank else 1
+    assert lib.mlora_linear_rows_plan(T, K, N, rank, n_mod, offs, flags | ops.W_PACKED | (ops.B_PACKED if rank else 0), v) == 0
+    return dict(zip(("passes", "grid", "groups", "multiplied", "kb", "slots"), list(v)))
+
+
+@pytest.mark.parametrize("silu", [False, True])
+@pytest.mark.parametrize("rank", [0, 16])
+@pytest.mark.parametrize("T", [1, 16, 17, 32])
+def test_whole_rows_are_dealt_exactly_once(T, rank, silu):
+    ops = load("ops")
+    unit = 2 if silu else 1
+    for N in (1184, 1200, 2048, 4096, 5120, 7008, 9600, 12288, 15360, 20112, 22016, 28416, 32000, 48000, 100000):
+        for K in (8, 72, 1032, 4096, 6144):
+            p = _rows_plan(T, K, N, ops.ANY_SUMS | (ops.SILU_MUL if silu else 0), rank=rank)
+            units = -(-N // (8 * unit))
+            if (N + 7) // 8 < 148 or T > 16 and units > 2 * (12 // unit) * 148:
+                assert p["passes"] == 0
+                continue
+            assert p["passes"] >= 1 and p["grid"] == min(148, units) and p["groups"] <= p["multiplied"] <= (12 if T > 16 else 20)
+            seen = []
+            for c in range(p["grid"]):  # the kernel's ranges, restated
+                u0, u1 = units * c // p["grid"], units * (c + 1) // p["grid"]
+                at = [(u0 + (u1 - u0) * i // p["passes"]) * unit for i in range(p["passes"] + 1)]
+                assert all(0 < b - a <= p["groups"] for a, b in zip(at, at[1:])) and at[0] == u0 * unit and at[-1] == u1 * unit
+                # a pass's groups are copied in three pieces at most, each inside a tile of 16
+                assert all((b - 1) // 16 - a // 16 < 3 for a, b in zip(at, at[1:]))
+                seen += range(at[0], at[-1])
+            assert seen == list(range(units * unit))
+            # what the ring, the sums and the adapters' side take fits the SM
+            rows = 32 if T > 16 else 16
+            slot = p["kb"] * (p["groups"] * 1024 + rows * 128)
+            assert 3 <= p["slots"] <= 16 and p["kb"] in (2, 4, 8)
+            assert p["slots"] * slot + 1024 * rows + 1024 + (rows * 400 if rank else 0) <= 227 * 1024 - 64
+
+
+def test_which_calls_get_whole_rows():
+    ops = load("ops")
+    some = ops.ANY_SUMS
+    taken = [(1, 16384, 4096), (4, 16384, 4096), (16, 8192, 2048), (17, 4096, 28416), (32, 6144, 4096), (16, 4096, 200000)]
+    left = [(33, 4096, 4096), (5, 8200, 4096), (16, 11008, 4096), (17, 6152, 4096), (32, 8192, 2048), (17, 4096, 28424), (8, 4096, 1176)]
+    assert all(_rows_plan(*c, some)["passes"] for c in taken) and not any(_rows_plan(*c, some)["passes"] for c in left)
+    for flags in (0, ops.STABLE_SUMS, ops.STABLE_SUMS | some):
+        assert not any(_rows_plan(*c, flags)["passes"] for c in taken)
+    # adapters: rank pitches of the packed layout, rows of shrink outputs that fit, modules of whole row tiles
+    assert all(_rows_plan(8, 4096, 4096, some, rank=r)["passes"] for r in (16, 32, 64, 128))
+    assert not any(_rows_plan(8, 4096, 4096, some, rank=r)["passes"] for r in (8, 24, 48))
+    assert _rows_plan(8, 4096, 12288, some, [0, 4096, 8192, 12288], 64)["passes"]
+    assert not _rows_plan(8, 4096, 12288, some, [0, 4096, 8192, 12288], 128)["passes"]
+    assert not _rows_plan(8, 4096, 12288, some, [0, 4096, 8200, 12288], 64)["passes"]
+    assert _rows_plan(8, 4096, 22016, some | ops.SILU_MUL, rank=64)["passes"] and not _rows_plan(8, 4096, 22016, some | ops.SILU_MUL, rank=128)["passes"]

@@ -1,4 +1,6 @@
 """The decode-size projection that gives every CTA whole output rows (``MLORA_ANY_SUMS``): against float64 and the stream-K kernel."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -12,8 +14,16 @@ def ops():
     return load("ops")
 
 
+def _plan(ops, T, K, N, flags, rank=0, n_mod=1, offs=None):
+    v, o = (C.c_int32 * 6)(), None if offs is None else (C.c_int32 * len(offs))(*offs)
+    assert load("_lib").lib().mlora_linear_rows_plan(T, K, N, rank, n_mod, o, flags | ops.ANY_SUMS | ops.W_PACKED | (ops.B_PACKED if rank else 0), v) == 0
+    return dict(zip(("passes", "grid", "groups", "multiplied", "kb", "slots"), list(v)))
+
+
 def _run(ops, cuda, T, K, N, flags=0, rank=0, n_mod=1, n_ad=5, seed=0, ids=None):
     """(output of this kernel, of stream-K, float64 reference, bound of one output's error)."""
+    offs = (0, N) if flags & ops.SILU_MUL or n_mod == 1 else tuple(N // 128 * i // n_mod * 128 for i in range(n_mod)) + (N,)
+    assert _plan(ops, T, K, N, flags, rank, n_mod, offs)["passes"], "another kernel than the one under test"
     g = torch.Generator().manual_seed(seed + T * 131 + K + N)
     x = torch.randn(T, K, generator=g).bfloat16()
     W = (torch.randn(N, K, generator=g) * K ** -0.5).bfloat16()
@@ -25,7 +35,6 @@ def _run(ops, cuda, T, K, N, flags=0, rank=0, n_mod=1, n_ad=5, seed=0, ids=None)
         B = (torch.randn(n_ad, N, pitch, generator=g) * 0.1).bfloat16()
         u = torch.randn(T, rank * n_mod, generator=g)
         slots = torch.randint(-1, n_ad + 1, (T,), generator=g).int() if ids is None else torch.tensor(ids).int()  # n_ad: no such adapter
-        offs = (0, N) if silu or n_mod == 1 else tuple(N // 128 * i // n_mod * 128 for i in range(n_mod)) + (N,)
         scales = torch.linspace(0.5, 2.0, n_ad)
         for t in range(T):
             s = int(slots[t])
@@ -62,12 +71,35 @@ def _check(got, old, want, f32):
     assert float(err.norm()) <= (1.0 if f32 else 1.01) * float(err_old.norm()) + 2 ** -20 * float(want.norm())
 
 
-@pytest.mark.parametrize("T", [1, 15, 16, 17, 32])
-@pytest.mark.parametrize("K,N", [(8, 1184), (72, 1200), (512, 2048), (1032, 4096), (4096, 7000), (4096, 9600), (4096, 12288), (3072, 20104), (4096, 28424),
-                                 (8192, 2048), (16384, 4096)])
-def test_plain(ops, cuda, T, K, N):
-    """One row group per CTA and several, one to three passes, odd numbers of k-blocks, ragged last rows, slots of 2 to 8 k-blocks."""
+@pytest.mark.parametrize("K,N,most", [(8, 1184, 32), (72, 1200, 32), (512, 2048, 32), (1032, 4096, 32), (4096, 7000, 32), (4096, 9600, 32), (4096, 12288, 32),
+                                      (3072, 20104, 32), (4096, 28416, 32), (4096, 28424, 16), (8192, 2048, 16), (16384, 4096, 4)])
+@pytest.mark.parametrize("T", [1, 4, 15, 16, 17, 32])
+def test_plain(ops, cuda, T, K, N, most):
+    """One row group per CTA and several, one and two passes, odd numbers of k-blocks, ragged last rows, slots of 2 to 8 k-blocks, up to
+    the ``most`` rows that are taken."""
+    if T > most:
+        assert not _plan(ops, T, K, N, ops.OUT_F32)["passes"]
+        return
     _check(*_run(ops, cuda, T, K, N, ops.OUT_F32), True)
+
+
+@pytest.mark.parametrize("T", [1, 16])
+@pytest.mark.parametrize("N", [48000, 72000])
+def test_three_passes_and_more(ops, cuda, T, N):
+    """Few enough columns that one CTA's rows are read in several passes: plain, SiLU*up, adapters with module boundaries inside a pass."""
+    assert _plan(ops, T, 72, N, 0)["passes"] == (3 if N == 48000 else 4)
+    _check(*_run(ops, cuda, T, 72, N, ops.OUT_F32), True)
+    _check(*_run(ops, cuda, T, 72, N, ops.SILU_MUL), False)
+    _check(*_run(ops, cuda, T, 136, N, ops.OUT_F32, 16, 8), True)
+    _check(*_run(ops, cuda, T, 72, N, ops.SILU_MUL, 32, 2), False)
+
+
+@pytest.mark.parametrize("T", [17, 32])
+def test_two_passes_beyond_16_rows(ops, cuda, T):
+    assert _plan(ops, T, 200, 28416, 0)["passes"] == 2 and _plan(ops, T, 200, 28416, ops.SILU_MUL)["passes"] == 2
+    _check(*_run(ops, cuda, T, 200, 28416, ops.SILU_MUL), False)
+    _check(*_run(ops, cuda, T, 200, 28416, ops.OUT_F32, 32, 3), True)
+    _check(*_run(ops, cuda, T, 200, 28416, ops.SILU_MUL, 16, 2), False)
 
 
 @pytest.mark.parametrize("T", [3, 32])
@@ -78,7 +110,7 @@ def test_activations_and_bf16(ops, cuda, T, flag, K, N):
 
 
 @pytest.mark.parametrize("T,rank,n_mod,K,N", [(1, 16, 1, 4096, 4096), (16, 16, 3, 1024, 12288), (17, 32, 3, 512, 1536), (32, 64, 3, 4096, 12288),
-                                              (32, 128, 1, 256, 1208), (9, 64, 1, 11008, 4096), (32, 16, 8, 128, 2048)])
+                                              (32, 128, 1, 256, 1208), (9, 64, 1, 8192, 4096), (4, 64, 1, 11008, 4096), (32, 16, 8, 128, 2048)])
 def test_adapters(ops, cuda, T, rank, n_mod, K, N):
     """Module boundaries inside a CTA's rows, adapters over several slots, rows without adapter or with one that does not exist."""
     _check(*_run(ops, cuda, T, K, N, ops.OUT_F32, rank, n_mod), True)
