@@ -36,8 +36,8 @@ class PagedCache:
         self.max_pages = min((per_seq + ps - 1) // ps + 1, self.n_pages)
         self.block_table = torch.zeros(self.max_batch, self.max_pages, dtype=torch.int32, device=self.device)
         self.seq_lens = torch.zeros(self.max_batch, dtype=torch.int32, device=self.device)
-        # host mirrors; device refreshes go through a fresh pinned staging tensor per copy, so a
-        # later host-side update can never race with an asynchronous copy still in the stream
+        # host mirrors; small device refreshes travel in launch parameters, larger ones through a fresh pinned staging tensor per
+        # copy: a later host-side update can never race with a refresh that is still in the stream
         self._bt_host = np.zeros((self.max_batch, self.max_pages), dtype=np.int32)
         self._len_host = np.zeros(self.max_batch, dtype=np.int32)
         self._free = list(range(self.n_pages - 1, -1, -1))

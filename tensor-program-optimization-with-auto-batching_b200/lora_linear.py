@@ -125,7 +125,8 @@ class MultiLoraLinear(nn.Module):
     # -- forward ---------------------------------------------------------------------------------------------
     def _slot_tensor(self, slots_per_batch_row, per_row, device):
         """int32 [rows] on the device: built once per (adapter list, tokens per row) and shared by every layer of
-        the model through the context -- one small host-to-device copy per generate step, not one per layer."""
+        the model through the context -- one upload per generate step (a launch that carries the list as parameters; a copy
+        beyond ``ops.PUT_AT_MOST`` requests), not one per layer."""
         key = (tuple(slots_per_batch_row), per_row, str(device))
         cache = self._ctx.slot_cache if self._ctx is not None else None
         if cache is not None and key in cache:
