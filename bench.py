@@ -15,6 +15,7 @@ token ids); nothing is read from outside this repository.
 from __future__ import annotations
 
 import argparse
+import ctypes
 import importlib
 import json
 import os
@@ -682,38 +683,51 @@ def kernel_rooflines(eng, pm, kv, B, slots, ops, torch, ctx, n_uniq, peak, reps=
             b += n_uniq * 2 * out_f * st.r_max + 4 * T + 4 * T * st.r_max * st.n_mod
         return b
 
-    def linears():
-        n, total = 0, 0
+    def takes_whole_rows(W, st, fl):
+        v, offs = (ctypes.c_int32 * 6)(), None
+        if st is not None and st.n_mod > 1 and not fl & ops.SILU_MUL:
+            offs = (ctypes.c_int32 * (st.n_mod + 1))(*st.mod_offsets)
+        fl |= ops.W_PACKED | (ops.B_PACKED if st is not None and st.b_packed else 0)
+        ops.check(ops._lib.lib().mlora_linear_rows_plan(T, W.shape[1], W.shape[0], st.r_max if st is not None else 0,
+                                                        st.n_mod if st is not None else 1, offs, fl, v), "mlora_linear_rows_plan")
+        return v[0] > 0
+
+    def linears():  # as the engine issues them
+        total, on = 0, {"linear_rows_kernel": 0, "linear_tc_kernel": 0}
         for lw in pm.layers:
             for W, key, src, dst, fl in ((lw.w_qkv, "qkv", x, qkv, 0), (lw.w_o, "o", attn, y, 0),
                                          (lw.w_gu, "gu", x, act, ops.SILU_MUL), (lw.w_down, "down", act, y, 0)):
-                st = lw.lora.get(key)
+                st, fl = lw.lora.get(key), fl | ops.ANY_SUMS
                 if st is not None:
                     ops.linear(src, W, st, sl, u=u_for(st), flags=fl, out=dst, work=eng.ws_linear)
-                else:  # as the engine issues it: same kernel variant as the LoRA projections around it
-                    ops.linear(src, W, flags=fl | ops.SHARE_LORA_KERNEL, out=dst, work=eng.ws_linear)
-                n += 1
+                else:
+                    fl |= ops.SHARE_LORA_KERNEL
+                    ops.linear(src, W, flags=fl, out=dst, work=eng.ws_linear)
+                on["linear_rows_kernel" if takes_whole_rows(W, st, fl) else "linear_tc_kernel"] += 1
                 total += lin_bytes(W, st, silu=bool(fl & ops.SILU_MUL))
-        ops.linear(x, pm.lm_head, flags=ops.OUT_F32 | ops.SHARE_LORA_KERNEL, out=eng.logits[:T], work=eng.ws_linear)
-        return n + 1, total + lin_bytes(pm.lm_head, None, out_f32=True)
+        fl = ops.OUT_F32 | ops.ANY_SUMS | ops.SHARE_LORA_KERNEL
+        ops.linear(x, pm.lm_head, flags=fl, out=eng.logits[:T], work=eng.ws_linear)
+        on["linear_rows_kernel" if takes_whole_rows(pm.lm_head, None, fl) else "linear_tc_kernel"] += 1
+        return on, total + lin_bytes(pm.lm_head, None, out_f32=True)
 
     def attentions():
         for l in range(pm.L):
             ops.paged_attention(qkv, kv.k_pages(l), kv.v_pages(l), kv.block_table, eng.row_slot[:T], eng.row_pos[:T],
                                 pm.Hq, pm.Hkv, pm.D, kv.page_size, pm.theta, True, out=attn, work=eng.ws_attn)
-        return pm.L, pm.L * (T * (ctx + 1) * 2 * pm.Hkv * pm.D * 2 + T * (pm.Hq + 2 * pm.Hkv) * pm.D * 2
+        return {"paged_attn_kernel": pm.L}, pm.L * (T * (ctx + 1) * 2 * pm.Hkv * pm.D * 2 + T * (pm.Hq + 2 * pm.Hkv) * pm.D * 2
                              + T * pm.Hq * pm.D * 2)
 
     eng.row_pos[:T].fill_(ctx)
     out = {}
     traffic = ncu_traffic()
-    for name, fn, kernel in (("linear", linears, "linear_tc_kernel"), ("attention", attentions, "paged_attn_kernel")):
+    for name, fn in (("linear", linears), ("attention", attentions)):
         side = torch.cuda.Stream()
         side.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(side):
-            n, total = fn()
+            on, total = fn()
         torch.cuda.current_stream().wait_stream(side)
         torch.cuda.synchronize()
+        n = sum(on.values())
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
             fn()
@@ -728,10 +742,10 @@ def kernel_rooflines(eng, pm, kv, B, slots, ops, torch, ctx, n_uniq, peak, reps=
         torch.cuda.synchronize()
         ms = e0.elapsed_time(e1) / reps
         achieved = total / (ms * 1e6)
-        out[name] = {"bound": "hbm", "kernel": kernel, "achieved": achieved, "peak": peak, "unit": "GB/s",
+        out[name] = {"bound": "hbm", "kernel": max(on, key=on.get), "launches_by_kernel": on, "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": peak_src + " copy bandwidth",
                      "launches": n, "avg_launch_us": 1e3 * ms / n, "algorithmic_bytes_per_launch": total / n,
-                     # DRAM read+write bytes per launch: ncu capture of one launch of this kernel at the benchmark's
+                     # DRAM read+write bytes per launch: ncu capture of one launch of ``kernel`` at the benchmark's
                      # shapes (profiles/), as a ratio to that launch's algorithmic bytes, applied to the step's
                      # average launch (traffic grows in proportion: the weights / KV pages dominate both)
                      "traffic": traffic[name][0] * total / n if name in traffic else None,
@@ -806,7 +820,7 @@ def run_kernel_case(which):
     if which in ("delta-step", "delta-chunk"):
         return run_delta_kernel_case(which, ops, dev, torch)
     if which == "linear":
-        # the q/k/v projection of one layer with its LoRA stack: 4 weight copies = 403 MB
+        # the q/k/v projection of one layer with its LoRA stack, as the engine issues it: 4 weight copies = 403 MB
         c = synth.operator_case(T, 4096, 12288, N_ADAPTERS, RANK, device=dev)
         Ws = [ops.PackedWeight((torch.randn(12288, 4096, device=dev) * 0.02).to(torch.bfloat16)) for _ in range(4)]
         A = torch.cat([c["A"]] * 3, 1).contiguous()
@@ -816,13 +830,13 @@ def run_kernel_case(which):
         u = ops.lora_shrink(c["x"], st, slots)
         out = torch.empty(T, 12288, dtype=torch.bfloat16, device=dev)
         for i in range(6):
-            ops.linear(c["x"], Ws[i % 4], st, slots, u=u, out=out)
+            ops.linear(c["x"], Ws[i % 4], st, slots, u=u, flags=ops.ANY_SUMS, out=out)
         # CUDA-event time of the same launch, warm, inside a graph (4 weight copies per replay)
         torch.cuda.synchronize()
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):
             for W in Ws:
-                ops.linear(c["x"], W, st, slots, u=u, out=out)
+                ops.linear(c["x"], W, st, slots, u=u, flags=ops.ANY_SUMS, out=out)
         for _ in range(3):
             g.replay()
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)

@@ -529,7 +529,8 @@ __global__ void __launch_bounds__(128, REP == 4 ? 2 : 4) paged_attn_group_kernel
 #pragma unroll
     for (int e = 0; e < 4; ++e) qf[j][e] = pack2(sq[j][dl * 8 + 2 * e], sq[j][dl * 8 + 2 * e + 1]);
 
-  // m, l: of the head whose scores this lane holds (l only this lane's share); acc: eight columns of every head
+  // m, l: of the head whose scores this lane holds (l only this lane's share, no number once a score was infinite or none); acc: eight
+  // columns of every head
   float m = -INFINITY, l = 0.f;
   f32x2 acc2[REP][4];
 #pragma unroll
@@ -569,7 +570,7 @@ __global__ void __launch_bounds__(128, REP == 4 ? 2 : 4) paged_attn_group_kernel
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int key = key0 + ((dl * R + r) & 7) * 2 + g;
-      p[r] = key < n_tok && key >= lo ? v[r] : -INFINITY;
+      p[r] = key < n_tok && key >= lo ? fmaf(v[r], 0.f, v[r]) : -INFINITY;  // (an infinite score is no number from here on)
       mx = fmaxf(mx, p[r]);
     }
 #pragma unroll
@@ -623,24 +624,31 @@ __global__ void __launch_bounds__(128, REP == 4 ? 2 : 4) paged_attn_group_kernel
     }
 
   // ---- merge the two lane groups of the warp, then the warps (+ the new token), and write -----------------
+  const auto leave = [&](float (&mj)[REP], float (&lj)[REP], float (&acc)[REP][8]) {
+#pragma unroll
+    for (int j = 0; j < REP; ++j) {
+      const float mo = __shfl_xor_sync(0xffffffffu, mj[j], 16), lo2 = __shfl_xor_sync(0xffffffffu, lj[j], 16);
+      float ao[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) ao[e] = __shfl_xor_sync(0xffffffffu, acc[j][e], 16);
+      merge_state(mj[j], lj[j], acc[j], mo, lo2, ao);
+      if (lane < 16) {
+        if (lane == 0) {
+          wm[warp][j] = mj[j];
+          wl[warp][j] = lj[j];
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) wacc[warp][j][lane * 8 + e] = acc[j][e];
+      }
+    }
+  };
 #pragma unroll
   for (int o = 1; o < LPH; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+  {
+    float mj[REP], lj[REP];
 #pragma unroll
-  for (int j = 0; j < REP; ++j) {
-    float mj = __shfl_sync(0xffffffffu, m, base + j * LPH), lj = __shfl_sync(0xffffffffu, l, base + j * LPH);
-    const float mo = __shfl_xor_sync(0xffffffffu, mj, 16), lo2 = __shfl_xor_sync(0xffffffffu, lj, 16);
-    float ao[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) ao[e] = __shfl_xor_sync(0xffffffffu, acc[j][e], 16);
-    merge_state(mj, lj, acc[j], mo, lo2, ao);
-    if (lane < 16) {
-      if (lane == 0) {
-        wm[warp][j] = mj;
-        wl[warp][j] = lj;
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) wacc[warp][j][lane * 8 + e] = acc[j][e];
-    }
+    for (int j = 0; j < REP; ++j) mj[j] = __shfl_sync(0xffffffffu, m, base + j * LPH), lj[j] = __shfl_sync(0xffffffffu, l, base + j * LPH);
+    leave(mj, lj, acc);
   }
   if (has_new && warp < REP) {
     float d = 0.f;
@@ -649,6 +657,59 @@ __global__ void __launch_bounds__(128, REP == 4 ? 2 : 4) paged_attn_group_kernel
     if (lane == 0) s_new[warp] = d;
   }
   __syncthreads();
+  // A head leaves out the keys that it scores -inf (and what is no number as long as it has seen no other), whatever their values are;
+  // a probability of 0 times such a value would be none.  Rows with such a score are rare: their warps walk the pages once more, key by
+  // key.  (The choice inside the walk above costs every row a tenth, and so does a function call here: 32 rows of 512 to 1024 keys 30.9 ->
+  // 34 us.)
+  bool odd = false;
+#pragma unroll
+  for (int w = 0; w < 4; ++w)
+#pragma unroll
+    for (int j = 0; j < REP; ++j) odd |= wl[w][j] != wl[w][j];
+  if (odd) {  // (uniform over the CTA)
+    __syncthreads();
+    int n2 = n_tok;
+    asm volatile("" : "+r"(n2));  // (the range again: kept, it would take registers from the walk above)
+    const int pages = (n2 + PS - 1) / PS, p0 = min(lo / PS, pages), each = (pages - p0 + a.n_splits - 1) / a.n_splits;
+    const int first = min(p0 + split * each, pages), last = min(first + each, pages);
+    float q[REP][8], mj[REP], lj[REP], acc[REP][8];
+#pragma unroll
+    for (int j = 0; j < REP; ++j) {
+      mj[j] = -INFINITY, lj[j] = 0.f;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) q[j][e] = sq[j][dl * 8 + e], acc[j][e] = 0.f;
+    }
+#pragma unroll 1
+    for (int s = first * SUB + warp; s < last * SUB; s += 4) {
+      const size_t at = place(s);
+#pragma unroll 1
+      for (int it = 0; it < IT; ++it) {
+        const int key = s * 16 + it * 2 + g;
+        const bool in = key < n_tok && key >= lo;
+        float k[8], v[8];
+        unpack8(ld_kv(a.k_pages + at + it * 2 * D, pol), k);
+        unpack8(ld_kv(a.v_pages + at + it * 2 * D, pol), v);
+#pragma unroll
+        for (int j = 0; j < REP; ++j) {
+          float d = 0.f;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) d = fmaf(q[j][e], k[e], d);
+#pragma unroll
+          for (int o = 8; o >= 1; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+          const float mn = fmaxf(mj[j], d);
+          if (in && d != -INFINITY && mn != -INFINITY) {
+            const float c = mj[j] == -INFINITY ? 0.f : exp2f(mj[j] - mn), p = exp2f(d - mn);
+            lj[j] = fmaf(lj[j], c, p);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) acc[j][e] = fmaf(acc[j][e], c, p * v[e]);
+            mj[j] = mn;
+          }
+        }
+      }
+    }
+    leave(mj, lj, acc);
+    __syncthreads();
+  }
 #pragma unroll
   for (int j = 0; j < REP; ++j) {
     const int h = h0 + j;
