@@ -63,7 +63,7 @@ extern "C" {
                                another order of fp32 sums is another choice at a near tie */
 #define MLORA_ANY_SUMS 2048 /* the caller does not need the sums over `in` in the order of mlora_linear_plan: up to 32 rows of
                                a packed weight may run on the kernel that gives every CTA whole output rows.  Which kernel that
-                               is changes with the rows (1..4, 5..16, 17..32), `in` and `out` (mlora_linear_rows_plan), so a
+                               is changes with the number of rows, `in` and `out` (mlora_linear_rows_plan), so a
                                row's last bits may depend on the size of its batch.  Without this flag, or with
                                MLORA_STABLE_SUMS, a call keeps the plan's sums, whose bits mlora_decode_chain reproduces */
 

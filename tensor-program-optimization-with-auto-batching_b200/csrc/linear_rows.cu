@@ -602,18 +602,50 @@ int plan_rows(const LinearArgs& a, void* work, cudaStream_t st) {
   }
 }
 
+// Up to which `in` a call is faster here than on stream-K, by rows and by the row groups of the widest CTA.  A k-block takes 0.11 us
+// however few groups a CTA has (two k16 steps of a product warp), stream-K's share of it falls with them: narrow projections of
+// great length lose what the missing hand-over gained.  Five groups multiply eight.  Above 16 rows x weighs as much as the weights.
+// Time here over stream-K's (CUDA events behind a norm, 148 SMs):
+//   in               1 row: 4096 8192 11008     4 rows: 2048 4096 8192     16 rows: 2048 4096 8192     32 rows: 2048 4096 6144
+//    2 groups (2048)        .89  1.06 1.09              .87  .97  1.21               .83  .96  1.16               .75  .84  .92
+//    4 groups (4096)        .89  .94  .94               .84  .98  1.05               .82  .89  .98                .82  .94  .99
+//    5 groups (5120)        .96  1.01 1.01              .99  1.06 1.10               .95  1.02 1.10               .88  .96  1.02
+//    6 groups (6144)        .90  .91  .91               .87  .95  .99                .89  .95  .98                .83  .91  .95
+//    7 groups (8192)        .86  .89  .89               .79  .92  .94                .85  .91  .93                .83  .87  .89
+//   11 groups (12288)       .87  .90  .91               .84  .91  .92                .87  .89  .91                .91  .93  .93
+// With rank-16 adapters 4 groups .92 at 4096 but 1.05 at 8192 with 1 row, .89 and .92 with 16, .93 at 4096 with 32; 6 groups 1.01 at 6144 with
+// 32; wider ranks gain more.  Within a column the limits lie where the slowest width of that many groups stays at 1.01 or below.
+int rows_in_limit(int T, int groups, bool lora) {
+  constexpr int any = 1 << 30;
+  static constexpr int plain[6][7] = {
+      // 1 group   2     3     4     5     6     7 and more
+      {5120, 6144, 6144, any, 6144, any, any},       // 1 row
+      {4096, 4096, 4096, 6144, 4096, any, any},      // 2
+      {3072, 3072, 3072, 4096, 2048, 8192, any},     // 3, 4
+      {3072, 3072, 3072, 4096, 2048, 8192, 8192},    // 5 to 7
+      {3072, 3072, 3072, 6144, 2048, 8192, 8192},    // 8 to 16
+      {6144, 6144, 4096, 4096, 5120, 6144, 6144}};   // 17 to 32
+  static constexpr int adapters[6][7] = {
+      {4096, 4096, 4096, 4096, 4096, any, any},
+      {4096, 4096, 4096, 8192, 4096, 8192, any},
+      {4096, 4096, 4096, 8192, 4096, 8192, any},
+      {4096, 4096, 4096, 8192, 4096, 8192, 8192},
+      {4096, 4096, 4096, 8192, 4096, 8192, 8192},
+      {3072, 3072, 3072, 4096, 4096, 4096, 6144}};
+  const int t = T <= 1 ? 0 : T <= 2 ? 1 : T <= 4 ? 2 : T <= 7 ? 3 : T <= 16 ? 4 : 5, g = groups < 7 ? groups - 1 : 6;
+  return lora ? adapters[t][g] : plain[t][g];
+}
+
 }  // namespace
 
 bool linear_rows_chosen(const LinearArgs& a) {
   if ((a.flags & (MLORA_ANY_SUMS | MLORA_STABLE_SUMS | MLORA_W_PACKED)) != (MLORA_ANY_SUMS | MLORA_W_PACKED) || a.T < 1 || a.T > 32) return false;
   // Fewer row groups than SMs leave SMs idle; stream-K cuts `in` for all of them (and has the shorter sums).
   if ((a.out + 7) / 8 < sm_count()) return false;
-  // With more rows, x and the products weigh as much as the weights where a CTA has few rows of great length, or passes over x
-  // three times.  Stream-K against this, us: 16 rows 11008 -> 4096 24.7 / 24.9; 32 rows 8192 -> 2048 20.1 / 20.3, 16384 -> 4096
-  // 38.4 / 41.7, 4096 -> 32000 47.6 / 49.5, but 4096 -> 16384 29.0 / 27.6, 4096 -> 22016 39.1 / 36.0.
-  if (a.in > (a.T <= 4 ? 1 << 30 : a.T <= 16 ? 8192 : 6144)) return false;
   const int unit = (a.flags & MLORA_SILU_MUL) ? 16 : 8;
-  if (a.T > 16 && (a.out + unit - 1) / unit > 2 * (RwCfg<32>::kMaxG * 8 / unit) * sm_count()) return false;
+  if (a.T > 16 && (a.out + unit - 1) / unit > 2 * (RwCfg<32>::kMaxG * 8 / unit) * sm_count()) return false;  // three passes over x
+  const int units = (a.out + unit - 1) / unit, grid = units < sm_count() ? units : sm_count();
+  if (a.in > rows_in_limit(a.T, (units + grid - 1) / grid * (unit / 8), a.u != nullptr)) return false;
   if (a.u == nullptr) return true;
   if (!(a.flags & MLORA_B_PACKED) || !aligned16(a.u) || a.r_max * a.n_mod > RwCfg<32>::kMaxRank) return false;
   if (!(a.r_max == 16 || a.r_max == 32 || a.r_max == 64 || a.r_max == 128)) return false;

@@ -165,6 +165,8 @@ def test_whole_rows_are_dealt_exactly_once(T, rank, silu):
             if (N + 7) // 8 < 148 or T > 16 and units > 2 * (12 // unit) * 148:
                 assert p["passes"] == 0
                 continue
+            if p["passes"] == 0 and K > 2048 and N < 7104:  # (by measurement: see the test below)
+                continue
             assert p["passes"] >= 1 and p["grid"] == min(148, units) and p["groups"] <= p["multiplied"] <= (12 if T > 16 else 20)
             seen = []
             for c in range(p["grid"]):  # the kernel's ranges, restated
@@ -185,11 +187,16 @@ def test_whole_rows_are_dealt_exactly_once(T, rank, silu):
 def test_which_calls_get_whole_rows():
     ops = load("ops")
     some = ops.ANY_SUMS
-    taken = [(1, 16384, 4096), (4, 16384, 4096), (16, 8192, 2048), (17, 4096, 28416), (32, 6144, 4096), (16, 4096, 200000)]
-    left = [(33, 4096, 4096), (5, 8200, 4096), (16, 11008, 4096), (17, 6152, 4096), (32, 8192, 2048), (17, 4096, 28424), (8, 4096, 1176)]
+    taken = [(1, 6144, 2048), (1, 16384, 4096), (2, 4096, 2048), (4, 16384, 8192), (4, 3072, 2048), (7, 4096, 4096), (8, 6144, 4096), (16, 2048, 5120), (16, 8192, 6144),
+             (17, 6144, 2048), (32, 4096, 4096), (32, 5120, 5120), (17, 4096, 28416), (32, 6144, 12288), (16, 4096, 200000)]
+    # (each of these was slower there than on stream-K, or was not measured)
+    left = [(1, 8192, 2048), (2, 8192, 2048), (4, 8192, 2048), (16, 8192, 2048), (4, 11008, 4096), (4, 4096, 5120), (5, 8192, 4096), (16, 5120, 5120), (16, 11008, 4096),
+            (5, 8200, 12288), (32, 6144, 3072), (32, 6144, 4096), (17, 6152, 12288), (32, 8192, 2048), (33, 4096, 4096), (17, 4096, 28424), (8, 4096, 1176)]
     assert all(_rows_plan(*c, some)["passes"] for c in taken) and not any(_rows_plan(*c, some)["passes"] for c in left)
     for flags in (0, ops.STABLE_SUMS, ops.STABLE_SUMS | some):
         assert not any(_rows_plan(*c, flags)["passes"] for c in taken)
+    assert _rows_plan(16, 8192, 4096, some, rank=16)["passes"] and not _rows_plan(1, 6144, 4096, some, rank=16)["passes"]
+    assert _rows_plan(32, 6144, 8192, some, rank=16)["passes"] and not _rows_plan(32, 6144, 6144, some, rank=16)["passes"]
     # adapters: rank pitches of the packed layout, rows of shrink outputs that fit, modules of whole row tiles
     assert all(_rows_plan(8, 4096, 4096, some, rank=r)["passes"] for r in (16, 32, 64, 128))
     assert not any(_rows_plan(8, 4096, 4096, some, rank=r)["passes"] for r in (8, 24, 48))
