@@ -514,6 +514,8 @@ def run_ours(args, rank, world, local_rank):
     torch.cuda.synchronize()
     prefill_s = time.perf_counter() - t0
 
+    for s in sids:  # (the page table's uploads are launches, but not a step's)
+        kv.reserve(s, kv.length(s) + total_steps + 1)
     launches0 = ops.launch_count()
     graph = eng.capture_decode(sids, slots, reserve_tokens=total_steps)
     launches_per_step = (ops.launch_count() - launches0) // 2  # one warm-up run + one capture
