@@ -8,16 +8,18 @@
 // narrow projection, through the same shared memory.
 //
 // Tokens are the M operand (16 per mma.sync m16n8k16) and a group of 8 weight rows the N operand: groups of 8 deal 4096 rows
-// evenly to 148 SMs, which tcgen05's 128-row tiles cannot, and sums in registers need no way through TMEM.  At 16 tokens the
-// products hide behind the stream; at 32 they and x cost up to a fifth of it.
+// evenly to 148 SMs, which 128-row tiles with the weights as M cannot, and sums in registers need no way through TMEM.  (tcgen05 with the
+// tokens as M would deal them as evenly; it was not built.)  The stream sets the pace, the products cost 1 us at one row and 9 to 16 % at
+// 32: without the mma.syncs (a copy that skips them) 4096 -> 12288 takes 18.3 / 19.6 / 20.7 us at 1 / 16 / 32 rows instead of
+// 19.4 / 21.0 / 22.6, 4096 -> 4096 12.1 instead of 14.4 at 32, 4096 -> 22016 SiLU*up 32.2 instead of 36.0.
 //
 // Measured behind a RMSNorm launch (CUDA events over a graph, us for both, stream-K -> this; the weights' bytes at 6458 GB/s):
 //              4096 -> 12288    4096 -> 4096    4096 -> 22016 SiLU*up    11008 -> 4096
-//    1 row     21.9 -> 18.9     12.5 -> 11.2    35.6 -> 30.1             23.3 -> 22.1
-//   16 rows    22.6 -> 20.0     13.3 -> 12.0    36.3 -> 31.1             24.7 -> 24.9 (not taken)
-//   32 rows    24.3 -> 22.6     15.5 -> 14.4    39.1 -> 36.0
+//    1 row     22.2 -> 19.4     12.6 -> 11.3    35.6 -> 30.2             23.3 -> 21.9
+//   16 rows    22.6 -> 21.0     13.3 -> 12.1    36.2 -> 31.8             24.7 -> 24.9 (not taken)
+//   32 rows    24.3 -> 22.6     15.4 -> 14.4    39.3 -> 36.0
 //   (bytes)    15.6             5.2             27.9                     14.0
-// with 16 adapters, behind a shrink, 32 rows: rank 16 4096 -> 12288 29.5 -> 27.6, 4096 -> 4096 18.2 -> 17.0; rank 64 52.5 -> 38.2, 32.4 -> 19.8.
+// with 16 adapters, behind a shrink, 32 rows: rank 16 4096 -> 12288 30.6 -> 28.4, 4096 -> 4096 17.9 -> 16.9; rank 64 56.1 -> 40.1, 31.3 -> 19.7.
 //
 // Warps: 0..7 products and output; 8, 9 copies (weights before the kernels in front have completed, token rows after); 10, 11
 // (LORA) list the batch's adapters and write scale * u as bf16.  A ring slot holds two to eight k-blocks of the CTA's weight rows
