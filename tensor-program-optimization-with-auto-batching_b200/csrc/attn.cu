@@ -369,8 +369,8 @@ __global__ void __launch_bounds__(128) paged_attn_kernel(AttnArgs a) {
 }
 
 // The same with REP query heads that share a key head in one CTA: its keys and values are read once instead of once per query
-// head.  (L2 gave them back, but that path was the limit: 32 heads over 8 key heads, 32 rows of 512 to 1024 keys 45.8 -> 32.0 us with
-// 15.5 us of bytes, of 8192 keys 410 -> 198 with 166.)  A page's REP x 8 scores of a lane group are summed over its 16 lanes by
+// head.  (L2 gave them back, but that path was the limit: 32 heads over 8 key heads, 32 rows of 512 to 1024 keys 45.8 -> 31.1 us with
+// 15.5 us of bytes, of 8192 keys 410 -> 193 with 166.)  A page's REP x 8 scores of a lane group are summed over its 16 lanes by
 // halving exchanges -- every step keeps half of the values -- so that each lane ends with REP / 2 of them and the exponentials are
 // taken once, not sixteen times.  The next page's keys are requested as soon as a page's scores are known, its values as soon
 // as they are summed up.  Two CTAs per SM at four heads: held to three (168 registers, spills) the same rows take 40.9 and 268 us; at two

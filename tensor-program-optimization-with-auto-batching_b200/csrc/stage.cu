@@ -3,8 +3,8 @@
 // A pinned buffer and a copy per table cost the host 25 to 60 us in front of a prompt pass's first kernel and the GPU a copy
 // engine's start for each; a launch costs 4 us and needs no buffer that has to outlive it.  Rows of a prompt pass go as one
 // record per sequence, not as three numbers per row.  With the engine's status words read at once and the stream's handle taken
-// without its object: two Llama layers, 2 prompts of 17 tokens 858 -> 711 us a pass, 5 of 17 to 301 1317 -> 1189; the
-// peft-style layer, 8 rows 68 -> 50.
+// without its object: two Llama layers, 2 prompts of 17 tokens 858 -> 711 us a pass, 5 of 17 to 301 1268 -> 1161; the
+// peft-style layer, 8 rows 68 -> 52 (570 -> 555 on the first pass over new inputs).
 #include "common.cuh"
 
 namespace mlora {
